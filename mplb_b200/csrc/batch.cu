@@ -1,7 +1,9 @@
 // Batched cavities behind the C ABI (mplbgpu_batch_*, include/mplbgpu.h).
 //
-// All cavities live in one pair of population arrays; a step advances every
-// active tile.  Steps run in chunks: either a CUDA graph that replays
+// All cavities live in one pair of population arrays.  Several steps of a
+// batch whose cavities fit keep strips of them in shared memory
+// (batch_resident.cuh); otherwise a step advances every active tile, and steps
+// run in chunks: either a CUDA graph that replays
 // `chunk` one-step launches, or one cooperative persistent launch of
 // `chunk` steps with a bounded grid barrier between steps (itself captured
 // in a graph when the driver allows it).  Every check period the moments
@@ -12,11 +14,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
 #include <string>
 #include <vector>
 
 #include "../../include/mplbgpu.h"
-#include "batch_kernels.cuh"
+#include "batch_resident.cuh"
 #include "lattice.h"
 
 using namespace mplb;
@@ -25,6 +28,18 @@ using namespace mplb;
 // floating-point contraction rules of their forms.
 extern template struct mplb::BatchLaunch<double>;
 extern template struct mplb::BatchLaunch<float>;
+extern template struct mplb::BatchResidentLaunch<double>;
+extern template struct mplb::BatchResidentLaunch<float>;
+
+// Resident strips launched together: the same cluster size, slots and block.
+struct ResidentClass {
+    int halves, ranks, warps;
+    int max_steps;      // per launch
+    bool whole;         // every strip is a whole cavity
+    long long work;     // nodes computed per step
+    std::vector<ResidentItem> items;
+    int first = 0;      // of its items in the device list
+};
 
 struct mplbgpu_batch {
     int precision = MPLBGPU_FP32_SHIFTED;
@@ -63,6 +78,17 @@ struct mplbgpu_batch {
     unsigned long long seed = 1;
     bool initialised = false;
     long long wait_limit = (long long)1 << 26;  // grid barrier polls
+    // resident strips of the active cavities (batch_resident.cuh); empty
+    // when a cavity is too large for them
+    std::vector<ResidentClass> resident;
+    ResidentItem* items = nullptr;
+    size_t items_cap = 0;
+    int sms = 1;
+    static constexpr int kSides = 5;   // side streams of the classes, made
+                                       // when a plan first needs them
+    cudaStream_t side[kSides] = {};
+    cudaEvent_t fork = nullptr;
+    cudaEvent_t join[kSides] = {};
     std::string err;
 };
 
@@ -133,7 +159,228 @@ int BuildTiles(mplbgpu_batch* b) {
     return MPLBGPU_OK;
 }
 
-// Active tiles and per-cavity tile ranges from b->active.
+// How the cavities of one side are held in shared memory.
+struct ResidentPlan {
+    int halves = 0, ranks = 1;
+    int strips = 1, overlap = 0;
+    double score = INFINITY;
+};
+
+// The best plan for cavities of side n when an SM has `load` nodes of the
+// active cavities to advance per step: the fewest SM cycles per node while
+// the GPU is full, the shortest step of one strip while it is not.  The
+// constants are measured on a B200: `fixed` is the part of a step that does
+// not shrink with its nodes (barrier, one pass' latency), `reload` the
+// reading and writing of a strip in steps of it, and the last table the share
+// of the SMs that clusters of that size can fill (a GPC's SMs are not always
+// a multiple of it).  Sweeps of every plan at sides 64-256 found none more than
+// 6 % faster than the one chosen here.
+ResidentPlan PlanResident(int n, bool f64, double load) {
+    static const int kRanks[] = {1, 2, 3, 4, 5, 6, 8, 9};
+    static const double kFill[] = {1.0, 1.0, 0.91, 0.89, 0.88, 0.89, 0.81,
+                                   0.91};
+    const double reload = f64 ? 1.3 : 2.5;
+    ResidentPlan best;
+    for (int halves = 0; halves < 3; halves++) {
+        const int cap = (f64 ? ResidentCap<double>() : ResidentCap<float>()) >>
+                        halves;
+        const double share = 1.0 / (1 << halves);
+        for (size_t r = 0; r < sizeof(kRanks) / sizeof(kRanks[0]); r++) {
+            const int ranks = kRanks[r];
+            const int most = ranks * (cap / n);   // rows of a strip
+            const double fixed = ranks > 1 ? 400 : 250;
+            auto consider = [&](int strips, int overlap, int rows) {
+                const double per_cta = (double)((rows + ranks - 1) / ranks) * n;
+                const double steps = strips > 1 ? overlap + 1 : 64;
+                const double cost = strips * ranks *
+                                    (per_cta + share * fixed) *
+                                    (1.0 + reload / steps) /
+                                    ((double)n * n * kFill[r]);
+                const double time = (per_cta + fixed) * (1.0 + reload / steps);
+                const double score =
+                    std::max(cost * load, time) + 0.1 * cost * load;
+                if (score >= best.score) return;
+                best.halves = halves;
+                best.ranks = ranks;
+                best.strips = strips;
+                best.overlap = overlap;
+                best.score = score;
+            };
+            if (most >= n) {
+                consider(1, 0, n);
+                continue;
+            }
+            for (int overlap : {3, 5, 7, 11, 15, 23}) {
+                const int inner = most - 2 * overlap;
+                if (inner < 1) break;
+                const int strips =
+                    std::max(2, (n - 2 * overlap + inner - 1) / inner);
+                const int valid = (n - 2 * overlap + strips - 1) / strips;
+                // the last strip takes what the others leave
+                if (n - overlap - (strips - 1) * valid < 1) continue;
+                consider(strips, overlap, valid + 2 * overlap);
+            }
+        }
+    }
+    return best;
+}
+
+// Resident strips of the active cavities, none if one does not fit.
+int BuildResident(mplbgpu_batch* b) {
+    const bool f64 = b->precision == MPLBGPU_FP64;
+    b->resident.clear();
+    double nodes = 0;
+    for (int c : b->active) {
+        const double n = b->cav[c].n;
+        // rows of up to an eighth of the slots: larger cavities keep the
+        // tile launches (a strip would be mostly overlap)
+        if (n * 8 > (f64 ? ResidentCap<double>() : ResidentCap<float>()))
+            return MPLBGPU_OK;
+        nodes += n * n;
+    }
+    const int group = f64 ? ResidentGroup<double>() : ResidentGroup<float>();
+    const long long unit = 128 / (f64 ? 8 : 4);
+    std::map<int, ResidentPlan> plans;
+    size_t count = 0;
+    for (int c : b->active) {
+        const int n = b->cav[c].n;
+        auto at = plans.find(n);
+        if (at == plans.end())
+            at = plans.emplace(n, PlanResident(n, f64, nodes / b->sms)).first;
+        const ResidentPlan& p = at->second;
+        const int valid = (n - 2 * p.overlap + p.strips - 1) / p.strips;
+        // the same block for all strips of a cavity: they read each other's
+        // rows of the launch before, so they stay in one class
+        const int tall = p.strips == 1 ? n : valid + 2 * p.overlap;
+        const int groups =
+            ((tall + p.ranks - 1) / p.ranks * n + group - 1) / group;
+        const int most = 24 >> p.halves;
+        const int passes = (groups + most - 1) / most;
+        const int warps = std::max(2, (groups + passes - 1) / passes);
+        const int max_steps = p.strips == 1 ? 128 : p.overlap + 1;
+        for (int j = 0; j < p.strips; j++) {
+            ResidentItem it{};
+            it.cav = c;
+            it.n = n;
+            it.base = (int)(b->hcav[c].base / unit);
+            it.whole = p.strips == 1;
+            const int v0 = j == 0 ? 0 : p.overlap + j * valid;
+            const int v1 = j + 1 == p.strips ? n : p.overlap + (j + 1) * valid;
+            it.row0 = std::max(0, v0 - p.overlap);
+            it.rows = std::min(n, v1 + p.overlap) - it.row0;
+            it.vrow0 = v0 - it.row0;
+            it.vrows = v1 - v0;
+            it.rows_per_cta = (it.rows + p.ranks - 1) / p.ranks;
+            ResidentClass* cls = nullptr;
+            for (ResidentClass& k : b->resident)
+                if (k.halves == p.halves && k.ranks == p.ranks &&
+                    k.warps == warps && k.max_steps == max_steps)
+                    cls = &k;
+            if (!cls) {
+                ResidentClass k{};
+                k.halves = p.halves;
+                k.ranks = p.ranks;
+                k.warps = warps;
+                k.max_steps = max_steps;
+                k.whole = it.whole != 0;
+                b->resident.push_back(k);
+                cls = &b->resident.back();
+            }
+            cls->items.push_back(it);
+            cls->work += (long long)it.rows * n;
+            count++;
+        }
+    }
+    // the longest class first; within a class the longest strips first
+    std::sort(b->resident.begin(), b->resident.end(),
+              [](const ResidentClass& x, const ResidentClass& y) {
+                  return x.work > y.work;
+              });
+    std::vector<ResidentItem> all;
+    for (ResidentClass& k : b->resident) {
+        std::stable_sort(k.items.begin(), k.items.end(),
+                         [](const ResidentItem& x, const ResidentItem& y) {
+                             return x.rows_per_cta * x.n >
+                                    y.rows_per_cta * y.n;
+                         });
+        k.first = (int)all.size();
+        all.insert(all.end(), k.items.begin(), k.items.end());
+    }
+    for (size_t k = 0; k + 1 < b->resident.size() && k < mplbgpu_batch::kSides;
+         k++) {
+        if (!b->fork)
+            BCK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+        if (!b->side[k])
+            BCK(cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking));
+        if (!b->join[k])
+            BCK(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
+    }
+    if (count > b->items_cap) {
+        BCK(cudaFree(b->items));
+        b->items = nullptr;
+        b->items_cap = 0;
+        BCK(cudaMalloc(&b->items, count * sizeof(ResidentItem)));
+        b->items_cap = count;
+    }
+    if (count > 0) {
+        BCK(cudaMemcpyAsync(b->items, all.data(),
+                            count * sizeof(ResidentItem),
+                            cudaMemcpyHostToDevice, b->stream));
+        BCK(cudaStreamSynchronize(b->stream));
+    }
+    return MPLBGPU_OK;
+}
+
+// nsteps (>= 4) steps of the active cavities in their resident strips.  A
+// whole cavity is stored where it was read; overlapping strips alternate
+// between the two arrays, an even number of times, so every field ends in
+// the array it started in.
+template <typename T>
+int AdvanceResident(mplbgpu_batch* b, long long nsteps, bool macro_last) {
+    const BatchDev d = MakeDev(b);
+    T* pop[2] = {static_cast<T*>(b->pop[b->cur]),
+                 static_cast<T*>(b->pop[1 - b->cur])};
+    const int lanes =
+        std::min<int>((int)b->resident.size(), mplbgpu_batch::kSides + 1);
+    if (lanes > 1) {
+        BCK(cudaEventRecord(b->fork, b->stream));
+        for (int k = 0; k < lanes - 1; k++)
+            BCK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
+    }
+    double busy[mplbgpu_batch::kSides + 1] = {};
+    for (const ResidentClass& k : b->resident) {
+        // to the stream that is free first: a class takes its share of the
+        // GPU's work, at least the time of its longest strip
+        const int lane = (int)(std::min_element(busy, busy + lanes) - busy);
+        const ResidentItem& longest = k.items.front();
+        busy[lane] += std::max((double)k.work / b->sms,
+                               (double)longest.rows_per_cta * longest.n + 400);
+        cudaStream_t st = lane == 0 ? b->stream : b->side[lane - 1];
+        const long long count =
+            k.whole ? (nsteps + k.max_steps - 1) / k.max_steps
+                    : 2 * ((nsteps + 2 * k.max_steps - 1) / (2 * k.max_steps));
+        for (long long l = 0; l < count; l++) {
+            const int n = (int)(nsteps * (l + 1) / count - nsteps * l / count);
+            const cudaError_t e = BatchResidentLaunch<T>::Run(
+                k.halves, k.ranks, k.warps, (int)k.items.size(), st, d, b->pc,
+                b->items + k.first, n, macro_last && l + 1 == count,
+                pop[k.whole ? 0 : (l & 1)], pop[k.whole ? 0 : 1 - (l & 1)]);
+            b->launches++;
+            if (e != cudaSuccess)
+                return BErr(b, MPLBGPU_ERR_CUDA,
+                            std::string("resident launch: ") +
+                                cudaGetErrorString(e));
+        }
+    }
+    for (int k = 0; k < lanes - 1; k++) {
+        BCK(cudaEventRecord(b->join[k], b->side[k]));
+        BCK(cudaStreamWaitEvent(b->stream, b->join[k], 0));
+    }
+    b->pc.seed += (uint32_t)nsteps;
+    return MPLBGPU_OK;
+}
+
+// Active tiles, per-cavity tile ranges and resident strips from b->active.
 int UploadActive(mplbgpu_batch* b) {
     std::vector<int4> ranges;
     int pos = 0;
@@ -153,7 +400,7 @@ int UploadActive(mplbgpu_batch* b) {
         BCK(cudaMemcpyAsync(b->ranges, ranges.data(), ranges.size() * sizeof(int4),
                             cudaMemcpyHostToDevice, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
-    return MPLBGPU_OK;
+    return BuildResident(b);
 }
 
 // One-step launches: one CTA per active tile (the hardware keeps the SMs
@@ -289,6 +536,16 @@ int CheckSync(mplbgpu_batch* b) {
 int Advance(mplbgpu_batch* b, long long nsteps, bool macro_last) {
     long long done = 0;
     const int chunk = std::max(2, b->tune.chunk);
+    // From 4 steps on a strip is worth reading into shared memory (and every
+    // launch of AdvanceResident has at least the two steps the kernel
+    // needs); persistent launches stay what the caller chose.
+    if (!b->tune.persistent && nsteps >= 4 && !b->resident.empty()) {
+        int rc = b->precision == MPLBGPU_FP64
+                     ? AdvanceResident<double>(b, nsteps, macro_last)
+                     : AdvanceResident<float>(b, nsteps, macro_last);
+        if (rc != MPLBGPU_OK) return rc;
+        done = nsteps;
+    }
     while (nsteps - done >= chunk) {
         const bool last = macro_last && nsteps - done == chunk;
         int rc = GraphChunk(b, last);
@@ -323,6 +580,12 @@ void FreeBatch(mplbgpu_batch* b) {
     cudaFree(b->sync_count);
     cudaFree(b->sync_gen);
     cudaFree(b->sync_err);
+    cudaFree(b->items);
+    for (int k = 0; k < mplbgpu_batch::kSides; k++) {
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+        if (b->join[k]) cudaEventDestroy(b->join[k]);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -407,6 +670,9 @@ mplbgpu_status mplbgpu_batch_create(const mplbgpu_cavity* cavities, int ncav,
     CRE(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     CRE(cudaEventCreate(&b->ev0));
     CRE(cudaEventCreate(&b->ev1));
+    int dev = 0;
+    CRE(cudaGetDevice(&dev));
+    CRE(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
     CRE(cudaMalloc(&b->dcav, ncav * sizeof(BatchCav)));
     CRE(cudaMemcpy(b->dcav, b->hcav.data(), ncav * sizeof(BatchCav),
                    cudaMemcpyHostToDevice));

@@ -66,11 +66,12 @@ __global__ void SumPartialKernel(const double* __restrict__ q, long long n,
 
 }  // namespace mplb
 
-#include "batch_kernels.cuh"
+#include "batch_resident.cuh"
 
 namespace mplb {
 
 template struct BatchLaunch<double>;
+template struct BatchResidentLaunch<double>;
 
 __global__ void BatchResidualPartialKernel(BatchDev bd,
                                            double* __restrict__ part) {

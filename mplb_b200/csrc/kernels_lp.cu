@@ -11,10 +11,11 @@ template struct Launch<3, __half>;
 
 }  // namespace mplb
 
-#include "batch_kernels.cuh"
+#include "batch_resident.cuh"
 
 namespace mplb {
 
 template struct BatchLaunch<float>;
+template struct BatchResidentLaunch<float>;
 
 }  // namespace mplb
