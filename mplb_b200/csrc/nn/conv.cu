@@ -33,6 +33,61 @@ __device__ __forceinline__ void TapOffset(int taps, int t, int& dh, int& dw) {
     }
 }
 
+// Bias, ReLU, mask and store of 16 output channels (n on) of one pixel.
+template <typename Args>
+__device__ __forceinline__ void StoreOutputs(const Args& a, long long pix,
+                                             int n, float* v,
+                                             const float* bias) {
+    if (a.bias != nullptr) {
+        const float4* b4 = reinterpret_cast<const float4*>(bias);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float4 b = b4[q];
+            v[4 * q] += b.x;
+            v[4 * q + 1] += b.y;
+            v[4 * q + 2] += b.z;
+            v[4 * q + 3] += b.w;
+        }
+    }
+    if (a.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i], 0.0f);
+    }
+    if (a.mask != nullptr) {
+        const uint4* m4 = reinterpret_cast<const uint4*>(
+            a.mask + pix * a.mask_ps + a.mask_coff + n);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const uint4 m = m4[q];
+            const uint32_t w[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                // bf16 > 0: sign bit clear and not +0
+                if ((w[e] & 0x8000u) || (w[e] & 0xFFFFu) == 0)
+                    v[8 * q + 2 * e] = 0.0f;
+                if ((w[e] & 0x80000000u) || (w[e] >> 16) == 0)
+                    v[8 * q + 2 * e + 1] = 0.0f;
+            }
+        }
+    }
+    if (a.out_f32) {
+        float4* o = reinterpret_cast<float4*>(
+            static_cast<float*>(a.out) + pix * a.out_ps + a.out_coff + n);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2],
+                               v[4 * q + 3]);
+    } else {
+        uint4* o = reinterpret_cast<uint4*>(
+            static_cast<__nv_bfloat16*>(a.out) + pix * a.out_ps +
+            a.out_coff + n);
+        o[0] = make_uint4(PackBf16(v[0], v[1]), PackBf16(v[2], v[3]),
+                          PackBf16(v[4], v[5]), PackBf16(v[6], v[7]));
+        o[1] = make_uint4(PackBf16(v[8], v[9]), PackBf16(v[10], v[11]),
+                          PackBf16(v[12], v[13]), PackBf16(v[14], v[15]));
+    }
+}
+
 }  // namespace
 
 template <int BK>
@@ -134,53 +189,187 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         TmemLoad16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
         const int n = n0 + c;
         if (!store || n >= a.cout) continue;
-        if (a.bias != nullptr) {
-            const float4* b4 = reinterpret_cast<const float4*>(a.bias + n);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float4 b = b4[q];
-                v[4 * q] += b.x;
-                v[4 * q + 1] += b.y;
-                v[4 * q + 2] += b.z;
-                v[4 * q + 3] += b.w;
+        StoreOutputs(a, pix, n, v, a.bias + n);
+    }
+
+    FenceBeforeSync();
+    __syncthreads();
+    if (warp == 2) {
+        FenceAfterSync();
+        TmemFree(tmem, a.tmem_cols);
+    }
+}
+
+// The 3x3 convolution of a band of tiles (see conv.cuh): the band's input
+// stays in shared memory for all nine taps.
+template <int BK>
+__global__ void __launch_bounds__(kConvThreads, 1)
+    ConvBandKernel(const __grid_constant__ CUtensorMap ta,
+                   const __grid_constant__ CUtensorMap tb, ConvBandArgs a) {
+    constexpr int SW = BK * 2;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = Align1024(smem_raw);
+    const uint32_t b_bytes = (uint32_t)a.bn * SW;   // weights of a k-block
+    const uint32_t stage_bytes = b_bytes * a.group;
+    uint8_t* ring = smem + a.chunks * a.chunk_bytes;
+    float* bias = reinterpret_cast<float*>(ring + a.stages * stage_bytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(bias + a.bn);
+    uint64_t* empty = full + a.stages;
+    uint64_t* a_full = empty + a.stages;
+    uint64_t* accum = a_full + a.chunks;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+    volatile int* cta_err = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int img = blockIdx.x / a.bands;
+    const int j0 = (int)(blockIdx.x - img * a.bands) * a.tiles;
+    const int nt = min(a.tiles, a.tiles_per_img - j0);
+    const int n0 = blockIdx.y * a.bn;
+    const int r0 = j0 * a.tile_step / a.pitch;   // the band's first image row
+    const int q0 = j0 * a.tile_step - r0 * a.pitch;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.stages; s++) {
+            BarInit(&full[s], 1);
+            BarInit(&empty[s], 1);
+        }
+        for (int c = 0; c < a.chunks; c++) BarInit(&a_full[c], 1);
+        BarInit(accum, 1);
+        *cta_err = 0;
+        FenceBarrierInit();
+        PrefetchTmap(&ta);
+        PrefetchTmap(&tb);
+    }
+    if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    for (int n = threadIdx.x; n < a.bn; n += kConvThreads)
+        bias[n] = a.bias != nullptr ? a.bias[n0 + n] : 0.0f;
+    FenceBeforeSync();
+    __syncthreads();
+    FenceAfterSync();
+    const uint32_t tmem = *tmem_slot;
+    const int nkb = 9 * a.chunks;
+    const int nst = (nkb + a.group - 1) / a.group;   // groups of k-blocks
+
+    if (warp == 0 && lane == 0) {
+        int c = 0, k0 = 0;   // slice and weight column of the k-block
+        int chunks = 0, st = 0;
+        for (; st < nst; st++) {
+            const int s = st % a.stages;
+            if (st >= a.stages &&
+                !BarWait(&empty[s], ((st / a.stages) + 1) & 1, cta_err)) {
+                Flag(cta_err, a.err);
+                break;
             }
-        }
-        if (a.relu) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i], 0.0f);
-        }
-        if (a.mask != nullptr) {
-            const uint4* m4 = reinterpret_cast<const uint4*>(
-                a.mask + pix * a.mask_ps + a.mask_coff + n);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const uint4 m = m4[q];
-                const uint32_t w[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    // bf16 > 0: sign bit clear and not +0
-                    if ((w[e] & 0x8000u) || (w[e] & 0xFFFFu) == 0)
-                        v[8 * q + 2 * e] = 0.0f;
-                    if ((w[e] & 0x80000000u) || (w[e] >> 16) == 0)
-                        v[8 * q + 2 * e + 1] = 0.0f;
+            const int blocks = min(a.group, nkb - st * a.group);
+            BarArriveExpectTx(&full[s], blocks * b_bytes);
+            for (int g = 0; g < blocks; g++) {
+                if (chunks < a.chunks) {
+                    BarArriveExpectTx(&a_full[chunks], a.box_bytes);
+                    TmaLoad4D(smem + chunks * a.chunk_bytes, &ta,
+                              &a_full[chunks], chunks * BK, -1, r0 - 1, img);
+                    chunks++;
+                }
+                TmaLoad2D(ring + s * stage_bytes + g * b_bytes, &tb, &full[s],
+                          k0 + c * BK, n0);
+                if (++c == a.chunks) {
+                    c = 0;
+                    k0 += a.cin;
                 }
             }
         }
-        if (a.out_f32) {
-            float4* o = reinterpret_cast<float4*>(
-                static_cast<float*>(a.out) + pix * a.out_ps + a.out_coff + n);
+        // every copy issued must land before exit
+        for (int i = 0; i < chunks; i++)
+            if (!BarWaitDrain(&a_full[i], 0)) Flag(cta_err, a.err);
+        for (int j = st > a.stages ? st - a.stages : 0; j < st; j++)
+            if (!BarWaitDrain(&full[j % a.stages], (j / a.stages) & 1))
+                Flag(cta_err, a.err);
+    } else if (warp == 1) {
+        // the whole warp walks the loop, one lane issues
+        const uint32_t idesc = InstrDescBf16(kTileM, a.bn, false, false);
+        constexpr uint32_t kHigh = SmemDescHigh(SW);
+        const uint32_t a0 = SmemDescLow(SmemAddr(smem)) + (q0 * SW >> 4);
+        const uint32_t b0 = SmemDescLow(SmemAddr(ring));
+        const uint32_t step = (uint32_t)(a.tile_step * SW) >> 4;
+        const uint32_t slice = (uint32_t)a.chunk_bytes >> 4;
+        const uint32_t row = (uint32_t)((a.pitch - 3) * SW) >> 4;
+        int kb = 0;
+        for (int st = 0, s = 0, phase = 0; st < nst; st++) {
+            bool ok = BarWait(&full[s], phase, cta_err);
+            const int blocks = min(a.group, nkb - kb);
+            for (int g = kb; g < min(kb + blocks, a.chunks); g++)
+                ok = ok && BarWait(&a_full[g], 0, cta_err);
+            if (!__all_sync(~0u, ok)) {
+                if (lane == 0) Flag(cta_err, a.err);
+                break;
+            }
+            FenceAfterSync();
+            uint32_t lb = b0 + (s * stage_bytes >> 4);
+            // the stage's first k-block: its slice, tap column and input
+            const int t = kb / a.chunks;
+            int c = kb - t * a.chunks, dw = t % 3;
+            uint32_t in = a0 + c * slice +
+                          ((uint32_t)((t / 3 * a.pitch + dw) * SW) >> 4);
+            if (ElectOne()) {
+                for (int g = 0; g < blocks; g++) {
+                    uint32_t la = in, d = tmem;
+                    for (int j = 0; j < nt; j++) {
 #pragma unroll
-            for (int q = 0; q < 4; q++)
-                o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2],
-                                   v[4 * q + 3]);
-        } else {
-            uint4* o = reinterpret_cast<uint4*>(
-                static_cast<__nv_bfloat16*>(a.out) + pix * a.out_ps +
-                a.out_coff + n);
-            o[0] = make_uint4(PackBf16(v[0], v[1]), PackBf16(v[2], v[3]),
-                              PackBf16(v[4], v[5]), PackBf16(v[6], v[7]));
-            o[1] = make_uint4(PackBf16(v[8], v[9]), PackBf16(v[10], v[11]),
-                              PackBf16(v[12], v[13]), PackBf16(v[14], v[15]));
+                        for (int k = 0; k < BK / 16; k++)
+                            Mma2(d, la + 2 * k, lb + 2 * k, kHigh, idesc,
+                                 (kb | g | k) != 0 ? 1u : 0u);
+                        la += step;
+                        d += a.bn;
+                    }
+                    lb += b_bytes >> 4;
+                    in += slice;
+                    if (++c == a.chunks) {
+                        c = 0;
+                        in -= slice * a.chunks - (SW >> 4);
+                        if (++dw == 3) {
+                            dw = 0;
+                            in += row;
+                        }
+                    }
+                }
+                Commit(&empty[s]);
+                if (st + 1 == nst) Commit(accum);
+            }
+            __syncwarp();
+            kb += blocks;
+            if (++s == a.stages) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+        if (kb < nkb && ElectOne()) Commit(accum);
+    }
+    __syncwarp();
+
+    const bool acc_ok = BarWaitDrain(accum, 0);
+    FenceAfterSync();
+    if (!acc_ok && threadIdx.x == 0) Flag(cta_err, a.err);
+    const bool store = acc_ok && *cta_err == 0;
+    for (int j = 0; j < nt; j++) {
+        const int q = (j0 + j) * a.tile_step + warp * 32 + lane;
+        const int y = q / a.pitch, x = q - y * a.pitch;
+        const bool pixel = store && x < a.W && y < a.H;
+        const long long pix = ((long long)img * a.H + y) * a.W + x;
+        const uint32_t t =
+            tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * a.bn);
+        int c = 0;
+        for (; c + 32 <= a.bn; c += 32) {
+            float v[32];
+            TmemLoad32(t + c, v);
+            if (pixel) {
+                StoreOutputs(a, pix, n0 + c, v, bias + c);
+                StoreOutputs(a, pix, n0 + c + 16, v + 16, bias + c + 16);
+            }
+            __syncwarp();
+        }
+        if (c < a.bn) {
+            float v[16];
+            TmemLoad16(t + c, v);
+            if (pixel) StoreOutputs(a, pix, n0 + c, v, bias + c);
         }
     }
 
@@ -448,6 +637,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // ---------------------------------------------------------------------------
 // Host side: tensor maps and launches.
 // ---------------------------------------------------------------------------
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -476,8 +666,8 @@ bool CheckView(const View& v, const char* what, std::string& err) {
     return ok;
 }
 
-bool EncodeAct(CUtensorMap* m, const View& v, int box_c, int swizzle,
-               std::string& err) {
+bool EncodeAct(CUtensorMap* m, const View& v, int box_c, int box_w, int box_h,
+               int swizzle, std::string& err) {
     EncodeTiledFn enc = Encoder();
     if (enc == nullptr) {
         err = "cuTensorMapEncodeTiled is not available";
@@ -488,8 +678,8 @@ bool EncodeAct(CUtensorMap* m, const View& v, int box_c, int swizzle,
     const cuuint64_t strides[3] = {(cuuint64_t)v.ps * 2,
                                    (cuuint64_t)v.ps * 2 * v.w,
                                    (cuuint64_t)v.ps * 2 * v.w * v.h};
-    const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)v.w,
-                               (cuuint32_t)(128 / v.w), 1};
+    const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)box_w,
+                               (cuuint32_t)box_h, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(
         m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, v.ptr, dims, strides, box,
@@ -502,6 +692,12 @@ bool EncodeAct(CUtensorMap* m, const View& v, int box_c, int swizzle,
         return false;
     }
     return true;
+}
+
+// Boxes of a 128-pixel tile.
+bool EncodeTile(CUtensorMap* m, const View& v, int box_c, int swizzle,
+                std::string& err) {
+    return EncodeAct(m, v, box_c, v.w, 128 / v.w, swizzle, err);
 }
 
 bool EncodeRows(CUtensorMap* m, const void* ptr, int rows, int kdim,
@@ -564,6 +760,127 @@ cudaError_t SetSmemAttr() {
     return e;
 }
 
+template <int BK>
+cudaError_t SetBandSmemAttr() {
+    static cudaError_t e =
+        cudaFuncSetAttribute(ConvBandKernel<BK>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSmemMax);
+    return e;
+}
+
+// How a 3x3 convolution is cut into bands; tiles == 0: tap by tap instead.
+struct BandPlan {
+    int tiles = 0;    // per CTA
+    int bn = 0;
+    int rows = 0;     // image rows of a band's input box
+    int group = 0;    // k-blocks of a weight stage
+    int stages = 0;
+    int smem = 0;
+};
+
+// Tiles and output channels of a CTA: two CTAs per SM of about 160
+// accumulator columns measured best over the network's layers (32 images,
+// cold L2, against tap by tap: 32 -> 32 channels at 128^2 31 us, was 48; 64 ->
+// 64 at 64^2 24, was 33; 128 -> 128 at 32^2 19, was 26), with fewer tiles and
+// then fewer channels while the GPU is not full.  Above 128 input channels the
+// band fills the shared memory that the weights stream through (192 -> 64 at
+// 64^2 64 us, was 61; 384 -> 128 at 32^2 108, was 53).
+BandPlan PlanBand(int nimg, int H, int W, int cin, int cout, int bk,
+                  int sm_count) {
+    BandPlan p;
+    if (cin > 128) return p;
+    const int pitch = W + 2, step = W == 128 ? pitch : 128;
+    const int per_img = W == 128 ? H : ((H - 1) * pitch + W + 127) / 128;
+    const int chunks = (cin + bk - 1) / bk, nkb = 9 * chunks;
+    int bn = 128;
+    while (cout % bn != 0) bn -= 16;
+    int tiles = std::max(1, std::min({4, (160 + bn / 2) / bn, per_img}));
+    const auto ctas = [&] {
+        return (long long)nimg * ((per_img + tiles - 1) / tiles) * (cout / bn);
+    };
+    while (tiles > 1 && ctas() < 2 * sm_count) tiles--;
+    while (bn % 32 == 0 && bn > 32 && ctas() < sm_count) bn /= 2;
+    for (; tiles >= 1; tiles--) {
+        const int rows = (W == 128 ? (tiles - 1) * step + 127
+                                   : pitch - 1 + (tiles - 1) * step + 127) /
+                             pitch + 3;
+        if (rows > 256) continue;
+        const int chunk = BandChunkBytes(rows, pitch, bk);
+        const int kb_bytes = bn * bk * 2;
+        for (int per_sm = 2; per_sm >= 1; per_sm--) {
+            const int room = std::min(kSmemPerSm / per_sm - 2048, kSmemMax);
+            const int left = room - BandSmemBytes(chunks, chunk, 0, 0, bn, bk);
+            if (left < std::min(3, nkb) * (kb_bytes + 16)) continue;
+            // Waiting for a stage, committing it and forming its addresses
+            // cost about 500 cycles, as much as 12 MMAs: a stage holds enough
+            // k-blocks for 32, or a third of what fits
+            const int mmas = tiles * (bk / 16);
+            p.group = std::min({nkb, (32 + mmas - 1) / mmas,
+                                std::max(1, left / 3 / (kb_bytes + 16))});
+            p.stages = std::min((nkb + p.group - 1) / p.group,
+                                left / (p.group * kb_bytes + 16));
+            p.tiles = tiles;
+            p.bn = bn;
+            p.rows = rows;
+            p.smem = BandSmemBytes(chunks, chunk, p.stages,
+                                   p.group * kb_bytes, bn, bk);
+            return p;
+        }
+    }
+    return p;
+}
+
+bool LaunchConvBand(const View& x, const void* w, const BandPlan& p, int bk,
+                    const float* bias, int relu, const View& y, bool y_f32,
+                    const View* mask, cudaStream_t stream, int* err_dev,
+                    std::string& err) {
+    ConvBandArgs a{};
+    a.H = x.h;
+    a.W = x.w;
+    a.pitch = x.w + 2;
+    a.tile_step = x.w == 128 ? a.pitch : 128;
+    a.tiles_per_img =
+        x.w == 128 ? x.h : ((x.h - 1) * a.pitch + x.w + 127) / 128;
+    a.tiles = p.tiles;
+    a.bands = (a.tiles_per_img + p.tiles - 1) / p.tiles;
+    a.cin = x.c;
+    a.chunks = (x.c + bk - 1) / bk;
+    a.chunk_bytes = BandChunkBytes(p.rows, a.pitch, bk);
+    a.box_bytes = (uint32_t)(p.rows * a.pitch * bk * 2);
+    a.cout = y.c;
+    a.bn = p.bn;
+    a.group = p.group;
+    a.stages = p.stages;
+    a.tmem_cols = Pow2Cols(p.tiles * p.bn);
+    a.out = y.ptr;
+    a.out_ps = y.ps;
+    a.out_f32 = y_f32 ? 1 : 0;
+    a.bias = bias;
+    a.relu = relu;
+    a.mask = mask ? static_cast<const __nv_bfloat16*>(mask->ptr) : nullptr;
+    a.mask_ps = mask ? mask->ps : 0;
+    a.err = err_dev;
+    CUtensorMap ta, tb;
+    if (!EncodeAct(&ta, x, bk, a.pitch, p.rows, bk * 2, err)) return false;
+    if (!EncodeRows(&tb, w, y.c, 9 * x.c, bk, p.bn, bk * 2, err)) return false;
+    const int smem = ResidencySafeSmem(p.smem, a.tmem_cols);
+    const dim3 grid(x.nimg * a.bands, y.c / p.bn);
+    cudaError_t e = bk == 64 ? SetBandSmemAttr<64>() : SetBandSmemAttr<32>();
+    if (e == cudaSuccess) {
+        if (bk == 64)
+            ConvBandKernel<64><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+        else
+            ConvBandKernel<32><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        err = std::string("convolution launch: ") + cudaGetErrorString(e);
+        return false;
+    }
+    return true;
+}
+
 cudaError_t SetWgradTSmemAttr() {
     static cudaError_t e = cudaFuncSetAttribute(
         WgradTKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
@@ -580,7 +897,8 @@ cudaError_t SetWgradSmemAttr() {
 
 bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
                 int relu, const View& y, bool y_f32, const View* mask,
-                cudaStream_t stream, int* err_dev, std::string& err) {
+                int sm_count, cudaStream_t stream, int* err_dev,
+                std::string& err) {
     if (!CheckView(x, "input", err) || !CheckView(y, "output", err))
         return false;
     if (mask != nullptr && !CheckView(*mask, "mask", err)) return false;
@@ -602,8 +920,16 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
         err = "output channels must be a multiple of 16";
         return false;
     }
+    // 1x1 convolutions have no rows to keep in shared memory
+    if (taps == 9) {
+        const BandPlan p =
+            PlanBand(x.nimg, x.h, x.w, x.c, y.c, bk, sm_count);
+        if (p.tiles > 0)
+            return LaunchConvBand(x, w, p, bk, bias, relu, y, y_f32, mask,
+                                  stream, err_dev, err);
+    }
     CUtensorMap ta, tb;
-    if (!EncodeAct(&ta, x, bk, bk * 2, err)) return false;
+    if (!EncodeTile(&ta, x, bk, bk * 2, err)) return false;
     if (!EncodeRows(&tb, w, y.c, taps * x.c, bk, bn, bk * 2, err)) return false;
     ConvArgs a{};
     a.H = x.h;
@@ -663,7 +989,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
     if (dy.c <= 64) {
         // few output channels: taps x input channels along M (WgradTKernel)
         CUtensorMap tx, tdy;
-        if (!EncodeAct(&tx, x, 32, 64, err) || !EncodeAct(&tdy, dy, 32, 64, err))
+        if (!EncodeTile(&tx, x, 32, 64, err) ||
+            !EncodeTile(&tdy, dy, 32, 64, err))
             return false;
         WgradTArgs t{};
         t.H = x.h;
@@ -702,7 +1029,7 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
         return true;
     }
     CUtensorMap ta, tb;
-    if (!EncodeAct(&ta, dy, 64, 128, err) || !EncodeAct(&tb, x, 64, 128, err))
+    if (!EncodeTile(&ta, dy, 64, 128, err) || !EncodeTile(&tb, x, 64, 128, err))
         return false;
     WgradArgs a{};
     a.H = x.h;

@@ -17,6 +17,21 @@
 // output gradient as X and the flipped, transposed weights
 // W'[c][8 - t][n] = W[n][t][c].
 //
+// ConvBandKernel is the 3x3 form for inputs that fit in shared memory.
+// Fetching each tap's box by itself moves the input nine times from L2 into
+// shared memory, which bound the layers of 32-64 channels.  Here a CTA takes a
+// band of tiles and loads the band's input rows once, with the pixel of halo on
+// every side (TMA's fill gives the padding): position q = y (W + 2) + x of a
+// slice of BK channels is row q of the buffer, so tap (dh, dw) of the tile
+// whose first output is at position q is the same buffer read from row
+// q + (dh + 1) (W + 2) + (dw + 1) on.  A tile is 128 consecutive positions; the
+// two columns of halo among them are computed and not stored (images of 128
+// columns step by W + 2 instead and have none).  The swizzle follows the
+// shared-memory address, so a tile may start at any row of the swizzle
+// pattern.  Weights stream through a ring, one (tap, slice) for all tiles of
+// the band.  Tap and slice follow each other as in ConvKernel, so the sums are
+// the same bits.
+//
 // WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
 // X[p + offset(t)][c]: M = 128 output channels, N = input channels, K = a
 // range of 128-pixel blocks (split over CTAs, accumulated with fp32 atomics).
@@ -63,6 +78,32 @@ struct ConvArgs {
     int* err;              // set to 1 when a wait gives up
 };
 
+struct ConvBandArgs {
+    int H, W;
+    int pitch;             // positions per image row: W + 2
+    int tile_step;         // positions between tiles
+    int tiles_per_img;
+    int tiles, bands;      // tiles of a band (CTA), bands of an image
+    int cin;
+    int chunks;            // BK-channel slices of the input
+    int chunk_bytes;       // shared memory of one slice of a band's input
+    uint32_t box_bytes;    // of its TMA box
+    int cout, bn;
+    int group;             // k-blocks (tap, slice) per stage of the weight ring
+    int stages;
+    int tmem_cols;
+    void* out;
+    long long out_ps;
+    int out_coff;
+    int out_f32;
+    const float* bias;
+    int relu;
+    const __nv_bfloat16* mask;
+    long long mask_ps;
+    int mask_coff;
+    int* err;
+};
+
 struct WgradArgs {
     int H, W, tiles_per_img, bh;
     int taps;
@@ -101,6 +142,11 @@ struct WgradTArgs {
 };
 
 template <int BK>
+__global__ void ConvBandKernel(const __grid_constant__ CUtensorMap ta,
+                               const __grid_constant__ CUtensorMap tb,
+                               ConvBandArgs a);
+
+template <int BK>
 __global__ void ConvKernel(const __grid_constant__ CUtensorMap ta,
                            const __grid_constant__ CUtensorMap tb,
                            ConvArgs a);
@@ -117,6 +163,16 @@ __global__ void WgradKernel(const __grid_constant__ CUtensorMap ta,
 // barriers).
 inline int ConvSmemBytes(int bk, int bn, int stages) {
     return 1024 + stages * (kTileM * bk * 2 + bn * bk * 2) + 256;
+}
+// ConvBandKernel: a slice of a band's input - the last tile reads up to two
+// positions past its rows - and the whole launch.
+inline int BandChunkBytes(int rows, int pitch, int bk) {
+    return ((rows * pitch + 2) * bk * 2 + 1023) / 1024 * 1024;
+}
+inline int BandSmemBytes(int chunks, int chunk_bytes, int stages,
+                         int stage_bytes, int bn, int bk) {
+    return 1024 + chunks * chunk_bytes + stages * (stage_bytes + 16) +
+           bn * 4 + 8 * chunks + 64;
 }
 inline int WgradSmemBytes(int b_atoms, int stages) {
     return 1024 + stages * ((2 + b_atoms) * 16384) + 256;

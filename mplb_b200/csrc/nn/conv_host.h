@@ -19,7 +19,8 @@ struct View {
 // shape or launch.  err_dev: device word the kernel sets on a timed-out wait.
 bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
                 int relu, const View& y, bool y_f32, const View* mask,
-                cudaStream_t stream, int* err_dev, std::string& err);
+                int sm_count, cudaStream_t stream, int* err_dev,
+                std::string& err);
 
 // dw[n][t][c] += sum_p dy[p][n] x[p + offset(t)][c].
 bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,

@@ -82,6 +82,31 @@ __device__ __forceinline__ void Mma(uint32_t d_tmem, uint64_t a_desc,
         : "memory");
 }
 
+// True in one lane of a converged warp.  Code that issues MMAs or commits runs
+// under this predicate: the compiler knows that one lane is left and forms the
+// operands (uniform registers) directly, where behind a test of the lane
+// number each MMA took over 100 cycles to issue.
+__device__ __forceinline__ bool ElectOne() {
+    uint32_t pred = 0, lane = 0;
+    asm volatile(
+        "{\n\t.reg .b32 %%rx;\n\t.reg .pred %%px;\n\t"
+        "elect.sync %%rx|%%px, %2;\n\t"
+        "@%%px mov.s32 %1, 1;\n\t"
+        "mov.s32 %0, %%rx;\n\t}"
+        : "+r"(lane), "+r"(pred)
+        : "r"(0xFFFFFFFFu));
+    return pred != 0;
+}
+
+// The same with the descriptors' two words apart (the high one, SmemDescHigh,
+// is a constant of both operands' layout).
+__device__ __forceinline__ void Mma2(uint32_t d_tmem, uint32_t a_low,
+                                     uint32_t b_low, uint32_t high,
+                                     uint32_t idesc, uint32_t accumulate) {
+    Mma(d_tmem, (uint64_t)high << 32 | a_low, (uint64_t)high << 32 | b_low,
+        idesc, accumulate);
+}
+
 // Arrives once on `bar` when every tcgen05 operation this thread issued so
 // far has completed.
 __device__ __forceinline__ void Commit(uint64_t* bar) {
@@ -108,6 +133,27 @@ __device__ __forceinline__ void TmemLoad16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// The same for 32 columns.
+__device__ __forceinline__ void TmemLoad32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
+        "%28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]),
+          "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+          "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+          "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // ---- descriptors -----------------------------------------------------------
 
 // swizzle_bytes: 128 or 64.  K-major: rows of `swizzle_bytes` along K, 8-row
@@ -125,6 +171,16 @@ __device__ __forceinline__ uint64_t SmemDesc(uint32_t saddr, uint32_t lbo,
     d |= 1ull << 46;
     d |= mode << 61;
     return d;
+}
+
+// The two words of a K-major descriptor: the low one holds the address, so
+// moving the operand by x bytes adds x / 16 to it.
+__device__ __forceinline__ uint32_t SmemDescLow(uint32_t saddr) {
+    return (saddr >> 4) & 0x3FFF;
+}
+__host__ __device__ constexpr uint32_t SmemDescHigh(int swizzle_bytes) {
+    return (uint32_t)(8 * swizzle_bytes >> 4) | (1u << 14) |
+           ((swizzle_bytes == 128 ? 2u : 4u) << 29);
 }
 
 __host__ __device__ constexpr uint32_t InstrDescBf16(int m, int n, bool a_mn,

@@ -495,7 +495,7 @@ int Conv(mplbnn_net* net, int l, const View& x, const View& y, bool y_f32) {
     std::string err;
     if (!LaunchConv(x, net->wf + net->w_off[l], s.taps,
                     net->params + net->b_off[l], s.relu, y, y_f32, nullptr,
-                    net->stream, net->err_dev, err))
+                    net->sm_count, net->stream, net->err_dev, err))
         return Fail(net, kInvalid, "layer " + std::to_string(l) + ": " + err);
     return kOK;
 }
@@ -505,7 +505,7 @@ int Dgrad(mplbnn_net* net, int l, const View& dz, const View& dx,
     const LayerSpec& s = kLayers[l];
     std::string err;
     if (!LaunchConv(dz, net->wd + net->w_off[l], s.taps, nullptr, 0, dx, false,
-                    mask, net->stream, net->err_dev, err))
+                    mask, net->sm_count, net->stream, net->err_dev, err))
         return Fail(net, kInvalid,
                     "data gradient of layer " + std::to_string(l) + ": " + err);
     return kOK;
@@ -721,6 +721,13 @@ int* PrimErrWord() {
     return w;
 }
 
+int SmCount() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 View FromAbi(const mplbnn_view* v) {
     return View{v->ptr, v->nimg, v->h, v->w, v->c, v->ps};
 }
@@ -762,7 +769,7 @@ int mplbnn_conv_forward(const mplbnn_view* x, const void* w, int taps,
     const View mv = mask ? FromAbi(mask) : View{};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (!LaunchConv(FromAbi(x), w, taps, bias, relu, FromAbi(y), y_f32 != 0,
-                    mask ? &mv : nullptr, s, errw, g_prim_error))
+                    mask ? &mv : nullptr, SmCount(), s, errw, g_prim_error))
         return kInvalid;
     return PrimFinish(s, errw);
 }
@@ -778,11 +785,8 @@ int mplbnn_conv_wgrad(const mplbnn_view* dy, const mplbnn_view* x, int taps,
         g_prim_error = "no device";
         return kCuda;
     }
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!LaunchWgrad(FromAbi(dy), FromAbi(x), taps, dw, sms, s, errw,
+    if (!LaunchWgrad(FromAbi(dy), FromAbi(x), taps, dw, SmCount(), s, errw,
                      g_prim_error))
         return kInvalid;
     return PrimFinish(s, errw);
