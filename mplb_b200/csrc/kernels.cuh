@@ -60,6 +60,28 @@ struct PhysConst {
     uint32_t seed;       // per launch (FP16 stochastic rounding)
 };
 
+// An operation of a LOCAL region's programme as the step kernels read it: a
+// CTA brings the operations of its row's three regions into shared memory
+// (StageWallOps) while its populations load.
+struct alignas(16) WallOp {
+    int kind;
+    uint32_t in, out, par;     // masks, as in RegionOp
+    union {
+        double denom;          // EQM, FP64
+        float fc[2];           // EQM, shifted forms: c0f, invf
+    };
+    const RegionOp* per_node;  // the operation itself where its constants
+                               // differ by node, else null
+    union {
+        double k[kMaxQ + 1];   // a of the parallel, b of the other populations
+        struct {
+            float kf[kMaxQ + 1];     // the same in FP32
+            float am1f[kMaxQ + 1];   // a - 1 of the parallel ones
+        };
+    };
+};
+constexpr int kRowOps = 3 * kMaxOps;   // operations staged by a CTA
+
 struct BlockDev {
     int n[3];
     int xoff;
@@ -95,6 +117,13 @@ struct BlockDev {
     // per region: class (bits 0-1) and fluid-like flag (bit 2); the pulled
     // and the stale populations (copies of RegionInfo::pull / ::stale)
     uint8_t rflags[kNumRegions];
+    // LOCAL regions' boundary programmes by region (kMaxOps operations each)
+    // and their lengths, and where their stale stores start (-1: none):
+    // addresses that follow from the region alone, so a node's operations
+    // load beside its populations instead of behind its region's record
+    uint8_t rnops[kNumRegions];
+    const WallOp* wops;
+    int rside[kNumRegions];
     uint32_t rpull[kNumRegions];
     uint32_t rstale[kNumRegions];
     // swap scheme (swap.cuh): per region the slots that live at slot opp(k)
@@ -652,45 +681,69 @@ __device__ __forceinline__ const RegionOp& NodeOp(const RegionOp& op, int x,
 }
 
 // EQMDiffuseRefl (KerCutCellEQMDiffuseRefl3D, Src/boundary_kernel.inc:
-// 1184-1276) with the wall constants precomputed per region.  Shifted
-// forms use sum_in f = sum_in h + sum_in w and w_opp(i) = w_i.
-template <typename L, typename T>
-__device__ __forceinline__ void ApplyEqm(typename Prec<T>::C* f,
-                                         const RegionOp& rop,
-                                         const PhysConst& pc, int x, int y,
-                                         int z) {
+// 1184-1276) with the wall constants precomputed per region: denom (FP64) or
+// c0 and inv (shifted forms, which use sum_in f = sum_in h + sum_in w and
+// w_opp(i) = w_i); k(i) and am1(i) the constants of population i.
+template <typename L, typename T, typename K, typename A>
+__device__ __forceinline__ void EqmWall(typename Prec<T>::C* f, uint32_t in,
+                                        uint32_t out, uint32_t par,
+                                        double denom, float c0, float inv,
+                                        const PhysConst& pc, K k, A am1) {
     constexpr int Q = L::Q;
-    const RegionOp& op = NodeOp(rop, x, y, z);
     if constexpr (Prec<T>::kShifted) {
         // rhoWall - 1 and w_i (rhoWall a_i - 1) without cancellation
         float sin = 0.0f;
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.in_mask >> i & 1u) sin += f[i];
-        const float drw = (op.c0f + 2.0f * sin) * op.invf;
+            if (in >> i & 1u) sin += f[i];
+        const float drw = (c0 + 2.0f * sin) * inv;
         const float rhoWall = 1.0f + drw;
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.par_mask >> i & 1u)
-                f[i] = pc.wf[i] * (op.am1f[i] + drw * op.af[i]);
+            if (par >> i & 1u) f[i] = pc.wf[i] * (am1(i) + drw * k(i));
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.out_mask >> i & 1u)
-                f[i] = f[L::opp(i)] + 2.0f * rhoWall * pc.wf[i] * op.bf[i];
+            if (out >> i & 1u)
+                f[i] = f[L::opp(i)] + 2.0f * rhoWall * pc.wf[i] * k(i);
     } else {
         double rhoIn = 0.0;
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.in_mask >> i & 1u) rhoIn = rhoIn + f[i];
-        const double rhoWall = (2.0 * rhoIn) / op.denom;
+            if (in >> i & 1u) rhoIn = rhoIn + f[i];
+        const double rhoWall = (2.0 * rhoIn) / denom;
+        // the products of the three weights, once
+        double wr[3], wr2[3];
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            wr[L::wclass(i)] = pc.w[i] * rhoWall;
+            wr2[L::wclass(i)] = (2.0 * rhoWall) * pc.w[i];
+        }
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.par_mask >> i & 1u) f[i] = (pc.w[i] * rhoWall) * op.a[i];
+            if (par >> i & 1u) f[i] = wr[L::wclass(i)] * k(i);
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (op.out_mask >> i & 1u)
-                f[i] = f[L::opp(i)] + ((2.0 * rhoWall) * pc.w[i]) * op.b[i];
+            if (out >> i & 1u) f[i] = f[L::opp(i)] + wr2[L::wclass(i)] * k(i);
     }
+}
+
+// The same from an operation in global memory, its node's own constants where
+// it has them.
+template <typename L, typename T>
+__device__ __forceinline__ void ApplyEqm(typename Prec<T>::C* f,
+                                         const RegionOp& rop,
+                                         const PhysConst& pc, int x, int y,
+                                         int z) {
+    using C = typename Prec<T>::C;
+    const RegionOp& op = NodeOp(rop, x, y, z);
+    EqmWall<L, T>(
+        f, op.in_mask, op.out_mask, op.par_mask, op.denom, op.c0f, op.invf, pc,
+        [&](int i) -> C {
+            const bool par = op.par_mask >> i & 1u;
+            if constexpr (Prec<T>::kShifted) return par ? op.af[i] : op.bf[i];
+            else return par ? op.a[i] : op.b[i];
+        },
+        [&](int i) { return op.am1f[i]; });
 }
 
 // FDPeriodic (KerCutCellPeriodic3D, Src/boundary_kernel.inc:1278-1666):
@@ -722,6 +775,76 @@ __device__ __forceinline__ void ApplyHbb(typename Prec<T>::C* f,
                                 : (typename P::C)op.b[i]);
 }
 
+// The operations of the regions rb, rb + 1, rb + 2 (a row's first node, middle
+// and last node) into shared memory: asynchronous copies that a CTA waits for
+// with its populations' loads under way.  Read one by one from global memory,
+// a wall node's constants took 2,300-3,500 cycles an operation and a node has
+// up to three (10,000-17,000 of a 3D wall node's 16,000-23,000 cycles, with no
+// other warp to cover them at the end of a launch).
+__device__ __forceinline__ void CpAsync16(void* smem, const void* gmem);
+__device__ __forceinline__ void CpAsyncCommit();
+template <int N>
+__device__ __forceinline__ void CpAsyncWait();
+
+__device__ __forceinline__ void StageWallOps(const BlockDev& b, int rb,
+                                             WallOp* s) {
+    constexpr int kPieces = kRowOps * (int)sizeof(WallOp) / 16;
+    const char* g = reinterpret_cast<const char*>(b.wops + rb * kMaxOps);
+    for (int e = threadIdx.x; e < kPieces; e += blockDim.x)
+        CpAsync16(reinterpret_cast<char*>(s) + 16 * e, g + 16 * e);
+    CpAsyncCommit();
+}
+
+// Whether a row of the regions rb .. rb + 2 has operations at its nodes
+// [x0, x0 + blockDim.x).
+__device__ __forceinline__ bool RowHasOps(const BlockDev& b, int rb, int x0) {
+    const int x1 = min(x0 + (int)blockDim.x, b.n[0]);
+    return (x0 == 0 && b.rnops[rb] != 0) ||
+           (x1 > 1 && x0 < b.n[0] - 1 && b.rnops[rb + 1] != 0) ||
+           (x1 == b.n[0] && b.rnops[rb + 2] != 0);
+}
+
+// The programme of one LOCAL node from its staged operations.
+template <typename L, typename T>
+__device__ __forceinline__ void ApplyWallOps(typename Prec<T>::C* f,
+                                             const WallOp* ops, int nops,
+                                             const PhysConst& pc,
+                                             const T* __restrict__ src,
+                                             const BlockDev& b, long long node,
+                                             int x, int y, int z) {
+    using P = Prec<T>;
+    using C = typename P::C;
+    constexpr int Q = L::Q;
+    for (int j = 0; j < nops; j++) {
+        const WallOp& op = ops[j];
+        const auto k = [&](int i) -> C {
+            if constexpr (P::kShifted) return op.kf[i];
+            else return op.k[i];
+        };
+        if (op.kind == kOpEqm) {
+            if (op.per_node != nullptr)
+                ApplyEqm<L, T>(f, *op.per_node, pc, x, y, z);
+            else
+                EqmWall<L, T>(f, op.in, op.out, op.par, op.denom, op.fc[0],
+                              op.fc[1], pc, k,
+                              [&](int i) { return op.am1f[i]; });
+        } else if (op.kind == kOpHbb) {
+            if (op.per_node != nullptr) {
+                ApplyHbb<L, T>(f, *op.per_node, pc, src, b, node, x, y, z);
+            } else {
+                const uint32_t out = op.out;
+#pragma unroll
+                for (int i = 0; i < Q; i++)
+                    if (out >> i & 1u)
+                        f[i] = P::Load(src, L::opp(i) * b.popstride + node,
+                                       L::opp(i), pc) + k(i);
+            }
+        } else if (op.kind == kOpZero) {
+            ApplyZero<L, T>(f, pc);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Fused step over one block.  kModeStep writes g^{n+1}; kModeMacro and
 // kModeF recompute the current f = post-boundary populations from the
@@ -738,7 +861,9 @@ __device__ __forceinline__ void ApplyHbb(typename Prec<T>::C* f,
 #ifndef MPLB_F64_MIN_BLOCKS
 #define MPLB_F64_MIN_BLOCKS 5
 #endif
-// One node of the step, any region class.
+// One node of the step, any region class.  Every thread of a CTA calls it
+// (`valid`: it has a node) with the CTA's staged operations; `staged`: they are
+// on their way and waited for here.
 template <int D, typename T, int MODE, bool O32>
 __device__ __forceinline__ void StepNode(const BlockDev& b,
                                          const PhysConst& pc,
@@ -748,7 +873,8 @@ __device__ __forceinline__ void StepNode(const BlockDev& b,
                                          double* __restrict__ out1,
                                          double* __restrict__ out2,
                                          double* __restrict__ out3, int x,
-                                         int y, int z) {
+                                         int y, int z, bool valid,
+                                         const WallOp* ops, bool staged) {
     using L = Lattice<D>;
     using P = Prec<T>;
     using C = typename P::C;
@@ -756,25 +882,14 @@ __device__ __forceinline__ void StepNode(const BlockDev& b,
     const int r = RegionOf(x, y, z, b.n, D);
     const int rf = b.rflags[r];
     const int cls = rf & 3;
-    if (cls == kDeferred) return;
+    valid = valid && cls != kDeferred;
     const long long node = NodeIndexT<D, O32>(b, x, y, z);
     C f[Q];
-    if (cls == kPure) {
-        if constexpr (O32) {
-            const T* ps = src + node;
-#pragma unroll
-            for (int i = 0; i < Q; i++)
-                f[i] = P::Load(ps, b.pull_off32[i], i, pc);
-        } else {
-#pragma unroll
-            for (int i = 0; i < Q; i++)
-                f[i] = P::Load(src, PullIndex<L>(b, node, i), i, pc);
-        }
-    } else {
+    if (valid) {
         // pull and stale masks from the kernel parameters, so the population
-        // loads do not wait for the region record
-        const uint32_t pull = b.rpull[r];
-        const uint32_t stale = b.rstale[r];
+        // loads wait for nothing else
+        const uint32_t pull = cls == kPure ? ~0u : b.rpull[r];
+        const uint32_t stale = cls == kPure ? 0u : b.rstale[r];
         const T* ps = src + node;
 #pragma unroll
         for (int i = 0; i < Q; i++) {
@@ -785,24 +900,32 @@ __device__ __forceinline__ void StepNode(const BlockDev& b,
                 f[i] = (C)0;
             }
         }
-        const RegionInfo& R = b.regions[r];
         if (stale) {
+            // node-major over the region's nodes (one layer on its boundary
+            // axes, the interior's extent on the others)
+            const int rx = r % 3, ry = (r / 3) % 3, rz = r / 9;
+            const int ex = rx == 1 ? b.n[0] - 2 : 1;
+            const int ey = ry == 1 ? b.n[1] - 2 : 1;
+            const int lx = rx == 1 ? x - 1 : 0, ly = ry == 1 ? y - 1 : 0;
+            const int lz = D == 3 && rz == 1 ? z - 1 : 0;
+            const int base = b.rside[r];
             const double* st =
-                b.stale + (R.side_base >= 0
-                               ? (R.side_base + LocalIndex(R, x, y, z)) * Q
-                               : 0);
+                b.stale +
+                (base >= 0 ? (base + ((long long)lz * ey + ly) * ex + lx) * Q
+                           : 0);
 #pragma unroll
             for (int i = 0; i < Q; i++)
                 if (stale >> i & 1u) f[i] = (C)st[i];
         }
-        for (int k = 0; k < R.nops; k++) {
-            const RegionOp& op = b.ops[R.op[k]];
-            if (op.kind == kOpEqm) ApplyEqm<L, T>(f, op, pc, x, y, z);
-            else if (op.kind == kOpHbb)
-                ApplyHbb<L, T>(f, op, pc, src, b, node, x, y, z);
-            else if (op.kind == kOpZero) ApplyZero<L, T>(f, pc);
-        }
     }
+    if (staged) {
+        CpAsyncWait<0>();
+        __syncthreads();
+    }
+    if (!valid) return;
+    if (cls != kPure)
+        ApplyWallOps<L, T>(f, ops + (r % 3) * kMaxOps, b.rnops[r], pc, src, b,
+                           node, x, y, z);
     const bool fl = (rf & 4) != 0;
     if (MODE == kModeF) {
         const long long dn =
@@ -844,12 +967,16 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
                T* __restrict__ dst, double* __restrict__ out0,
                double* __restrict__ out1, double* __restrict__ out2,
                double* __restrict__ out3) {
+    __shared__ WallOp ops[kRowOps];
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     const int z = D == 3 ? (int)blockIdx.z : 0;
-    if (x >= b.n[0]) return;
-    StepNode<D, T, MODE, O32>(b, pc, src, dst, out0, out1, out2, out3, x, y,
-                              z);
+    const int rb = RegionOf(0, y, z, b.n, D);
+    const bool staged = RowHasOps(b, rb, blockIdx.x * blockDim.x);
+    if (staged) StageWallOps(b, rb, ops);
+    StepNode<D, T, MODE, O32>(b, pc, src, dst, out0, out1, out2, out3,
+                              min(x, b.n[0] - 1), y, z, x < b.n[0], ops,
+                              staged);
 }
 
 // Interior nodes per thread (G, 32 apart along x): all G nodes' loads are
@@ -1156,8 +1283,9 @@ __device__ __forceinline__ void PureNodeGroup(const BlockDev& b,
 constexpr int kSplitRows = 64;
 constexpr int kSplitCta = 128;   // threads per CTA of SplitStepKernel
 constexpr int kSplitWarps = kSplitCta / 32;
+static_assert(2 * kSplitRows == kSplitCta, "one x-face node per thread");
 
-// Staged interior of the shifted forms.  Each warp takes kStageTasks
+// Staged interior of the shifted forms.  Each warp takes up to kStageTasks
 // consecutive 64-node row segments and runs them through a pipeline of
 // StageDepth<T>() shared-memory stages: while it computes one segment, the
 // copies of the next segments' 19 source windows are in flight (16-byte
@@ -1223,12 +1351,13 @@ __device__ __forceinline__ SplitTask InteriorTask(const BlockDev& b,
 }
 
 // CTAs of one chunk: the x-face CTA and the interior CTAs (a warp takes
-// one task, or kStageTasks with the staged interior).
+// one task, or `tasks` <= kStageTasks with the staged interior).
 template <int G, bool STAGED = false>
-__host__ __device__ constexpr long long SplitChunkCtas(int n0) {
+__host__ __device__ constexpr long long SplitChunkCtas(int n0,
+                                                       int tasks = 1) {
     return 1 + ((long long)kSplitRows * ((n0 + 32 * G - 1) / (32 * G)) +
-                kSplitWarps * (STAGED ? kStageTasks : 1) - 1) /
-                   (kSplitWarps * (STAGED ? kStageTasks : 1));
+                kSplitWarps * (STAGED ? tasks : 1) - 1) /
+                   (kSplitWarps * (STAGED ? tasks : 1));
 }
 
 __device__ __forceinline__ void CpAsync16(void* smem, const void* gmem) {
@@ -1246,15 +1375,15 @@ __device__ __forceinline__ void CpAsyncWait() {
 }
 
 // The staged interior of one CTA of a chunk (see StagedStep): warp k takes
-// the chunk's tasks (w - 1) kSplitWarps kStageTasks + k kStageTasks + t,
-// t < kStageTasks (task -> row t / tasks per row, segment t % tasks per
+// the chunk's tasks (w - 1) kSplitWarps tasks + k tasks + t, t < tasks (task -> row t / tasks per row, segment t % tasks per
 // row).  Lane l computes the pair l, l + 32 of the segment (PairFinish).
 template <int D, typename T, bool O32>
 __device__ __forceinline__ void StagedInterior(const BlockDev& b,
                                                const PhysConst& pc,
                                                const T* __restrict__ src,
                                                T* __restrict__ dst, int chunk,
-                                               int w, int rows, int ny) {
+                                               int w, int rows, int ny,
+                                               int tasks) {
     using L = Lattice<D>;
     constexpr int Q = L::Q;
     constexpr int S = StageDepth<T>();
@@ -1266,12 +1395,12 @@ __device__ __forceinline__ void StagedInterior(const BlockDev& b,
     const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
     T* stages = reinterpret_cast<T*>(stage_raw) + warp * S * Q * kWin;
     const int tpr = (b.n[0] + 63) / 64;
-    const int t0 = ((w - 1) * kSplitWarps + warp) * kStageTasks;
+    const int t0 = ((w - 1) * kSplitWarps + warp) * tasks;
     // task t of this warp: its row (or -1) and first column
     auto task = [&](int t, int& r, int& xs) {
         const int g = t0 + t;
         const int rl = g / tpr;
-        r = (t < kStageTasks && rl < kSplitRows &&
+        r = (t < tasks && rl < kSplitRows &&
              chunk * kSplitRows + rl < rows)
                 ? chunk * kSplitRows + rl
                 : -1;
@@ -1298,7 +1427,7 @@ __device__ __forceinline__ void StagedInterior(const BlockDev& b,
     };
 #pragma unroll
     for (int t = 0; t < S - 1; t++) issue(t, t);
-    for (int t = 0; t < kStageTasks; t++) {
+    for (int t = 0; t < tasks; t++) {
         issue(t + S - 1, (t + S - 1) % S);
         CpAsyncWait<S - 1>();
         __syncwarp();
@@ -1329,6 +1458,8 @@ __device__ __forceinline__ void StagedInterior(const BlockDev& b,
     }
 }
 
+constexpr unsigned kWallsFirst = ~0u;   // CTA order of SplitStepKernel
+
 // The step with no warp mixing interior and boundary nodes (a warp holding
 // one boundary node runs that node's boundary programme with the other 31
 // lanes idle: at 128^3 a third of the issue slots had no work).  One launch,
@@ -1349,7 +1480,9 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
                                            ? MPLB_F64_MIN_BLOCKS
                                            : MPLB_LP_MIN_BLOCKS)
     SplitStepKernel(BlockDev b, PhysConst pc, const T* __restrict__ src,
-                    T* __restrict__ dst, unsigned blk0, unsigned spc) {
+                    T* __restrict__ dst, unsigned blk0, unsigned spc,
+                    int tasks) {
+    __shared__ WallOp ops[kRowOps];
     // block and row counts fit in 32 bits (the launcher checks the grid),
     // so the index arithmetic stays 32-bit
     const int nbx = (b.n[0] + (int)blockDim.x - 1) / (int)blockDim.x;
@@ -1358,29 +1491,49 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
     const unsigned nsr = (unsigned)nbx * (2 * nz + (D == 3 ? 2 * ny : 0));
     constexpr int G = SplitGroup<T>();
     constexpr bool kStaged = StagedStep<T>();
-    const unsigned per_chunk = (unsigned)SplitChunkCtas<G, kStaged>(b.n[0]);
+    const unsigned per_chunk = (unsigned)SplitChunkCtas<G, kStaged>(b.n[0], tasks);
     // CTA order: spc = 0, the shell rows first, then the chunks (blk0: a
-    // launch of the chunks alone starts after the shell rows); spc > 0, each
-    // chunk's CTAs followed by spc shell-row CTAs, so the shell rows' long
-    // boundary programmes run beside interior CTAs instead of in waves of
+    // launch of the chunks alone starts after the shell rows);
+    // spc = kWallsFirst, the shell rows, every chunk's x-face CTA, then the
+    // interior CTAs: a wall node's programme takes longer than an interior
+    // CTA, and started last it would be alone at the end of a small launch;
+    // else each chunk's CTAs followed by spc shell-row CTAs, so that the shell
+    // rows' long programmes run beside interior CTAs instead of in waves of
     // their own at the start
-    unsigned blk;
-    if (spc > 0) {
-        const unsigned slot = blockIdx.x / (per_chunk + spc);
-        const unsigned r = blockIdx.x - slot * (per_chunk + spc);
-        if (r >= per_chunk) {
-            blk = slot * spc + (r - per_chunk);
-            if (blk >= nsr) return;
-        } else {
-            blk = nsr + slot * per_chunk + r;
+    unsigned blk, chunk_w = 0, chunk_c = 0;
+    if (spc == kWallsFirst) {
+        const int all = ny * (D == 3 ? b.n[2] - 2 : 1);
+        const unsigned chunks = (unsigned)((all + kSplitRows - 1) / kSplitRows);
+        blk = blockIdx.x;
+        if (blk >= nsr) {
+            chunk_c = blk - nsr;
+            if (chunk_c >= chunks) {
+                chunk_w = 1 + (chunk_c - chunks) % (per_chunk - 1);
+                chunk_c = (chunk_c - chunks) / (per_chunk - 1);
+            }
         }
     } else {
-        blk = blockIdx.x + blk0;
+        if (spc > 0) {
+            const unsigned slot = blockIdx.x / (per_chunk + spc);
+            const unsigned r = blockIdx.x - slot * (per_chunk + spc);
+            if (r >= per_chunk) {
+                blk = slot * spc + (r - per_chunk);
+                if (blk >= nsr) return;
+            } else {
+                blk = nsr + slot * per_chunk + r;
+            }
+        } else {
+            blk = blockIdx.x + blk0;
+        }
+        if (blk >= nsr) {
+            chunk_c = (blk - nsr) / per_chunk;
+            chunk_w = (blk - nsr) % per_chunk;
+        }
     }
     if (blk < nsr) {
         const int row = (int)(blk / nbx);
-        const int x = (int)(blk % nbx) * blockDim.x + threadIdx.x;
-        if (x >= b.n[0]) return;
+        const int x0 = (int)(blk % nbx) * blockDim.x;
+        const int x = x0 + threadIdx.x;
         int y, z;
         if (row < 2 * nz) {
             y = (row & 1) ? b.n[1] - 1 : 0;
@@ -1390,25 +1543,31 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
             z = (r2 & 1) ? b.n[2] - 1 : 0;
             y = 1 + (r2 >> 1);
         }
-        StepNode<D, T, kModeStep, O32>(b, pc, src, dst, nullptr, nullptr,
-                                       nullptr, nullptr, x, y, z);
+        const int rb = RegionOf(0, y, z, b.n, D);
+        const bool staged = RowHasOps(b, rb, x0);
+        if (staged) StageWallOps(b, rb, ops);
+        StepNode<D, T, kModeStep, O32>(
+            b, pc, src, dst, nullptr, nullptr, nullptr, nullptr,
+            min(x, b.n[0] - 1), y, z, x < b.n[0], ops, staged);
         return;
     }
-    blk -= nsr;
     const int rows = ny * (D == 3 ? b.n[2] - 2 : 1);
-    const int chunk = (int)(blk / per_chunk);
-    const int w = (int)(blk % per_chunk);
+    const int chunk = (int)chunk_c, w = (int)chunk_w;
     if (w == 0) {
-        const int r = chunk * kSplitRows + (int)(threadIdx.x >> 1);
-        if (threadIdx.x >= 2 * kSplitRows || r >= rows) return;
+        const int r =
+            min(chunk * kSplitRows + (int)(threadIdx.x >> 1), rows - 1);
         const int x = (threadIdx.x & 1) ? b.n[0] - 1 : 0;
-        StepNode<D, T, kModeStep, O32>(b, pc, src, dst, nullptr, nullptr,
-                                       nullptr, nullptr, x, 1 + r % ny,
-                                       D == 3 ? 1 + r / ny : 0);
+        constexpr int rb = 12;   // interior rows: the x faces are 12 and 14
+        const bool staged = (b.rnops[rb] | b.rnops[rb + 2]) != 0;
+        if (staged) StageWallOps(b, rb, ops);
+        StepNode<D, T, kModeStep, O32>(
+            b, pc, src, dst, nullptr, nullptr, nullptr, nullptr, x, 1 + r % ny,
+            D == 3 ? 1 + r / ny : 0,
+            chunk * kSplitRows + (int)(threadIdx.x >> 1) < rows, ops, staged);
         return;
     }
     if constexpr (kStaged) {
-        StagedInterior<D, T, O32>(b, pc, src, dst, chunk, w, rows, ny);
+        StagedInterior<D, T, O32>(b, pc, src, dst, chunk, w, rows, ny, tasks);
     } else {
         const SplitTask k = InteriorTask<G>(b, chunk, w);
         if (k.r < 0 || k.r >= rows) return;

@@ -15,7 +15,7 @@ static_assert(StageSmemBytes<3, __half>() <= 48 * 1024,
 // StagedStep<T>()) or SplitSwapKernel (never staged) for block b (0: too
 // many).
 template <int D, typename T, bool STAGED = StagedStep<T>()>
-long long SplitBlocks(const BlockDev& b) {
+long long SplitBlocks(const BlockDev& b, int tasks) {
     const long long nbx = (b.n[0] + kStepThreads - 1) / kStepThreads;
     const long long ny = b.n[1] - 2;
     const long long nz = D == 3 ? b.n[2] : 1;
@@ -23,7 +23,7 @@ long long SplitBlocks(const BlockDev& b) {
     const long long nsr = nbx * (2 * nz + (D == 3 ? 2 * ny : 0));
     const long long chunks = (rows + kSplitRows - 1) / kSplitRows;
     const long long blocks =
-        nsr + chunks * SplitChunkCtas<SplitGroup<T>(), STAGED>(b.n[0]);
+        nsr + chunks * SplitChunkCtas<SplitGroup<T>(), STAGED>(b.n[0], tasks);
     return blocks > 0x7fffffffLL ? 0 : blocks;
 }
 
@@ -36,11 +36,37 @@ long long SplitShellBlocks(const BlockDev& b) {
     return nbx * (2 * nz + (D == 3 ? 2 * ny : 0));
 }
 
+// Whether a step starts with the boundary nodes (kWallsFirst): while both
+// population arrays stay in the L2 cache (126 MB), where it takes 64^3 from
+// 20.5 to 16.8 us in FP64 and 96^3 from 39.9 to 36.4 in FP16.  Beyond that the
+// x faces have to run next to their rows, or the sectors they share are read
+// and written twice in HBM (128^3 in FP64 140 us against 114).
+template <typename T>
+bool WallsFirst(const BlockDev& b, int q) {
+    return 2.0 * q * (double)b.popstride * sizeof(T) <= 100e6;
+}
+
+// Row segments a warp of the staged interior takes one after the other: up to
+// kStageTasks, fewer while the GPU's warps are not all busy (24^3 in FP16 is
+// three segments deep with one each, and took 12.3 us with eight).
+template <int D, typename T>
+int StageTasks(const BlockDev& b) {
+    if (!StagedStep<T>()) return 1;
+    const long long segments = (long long)(b.n[1] - 2) *
+                               (D == 3 ? b.n[2] - 2 : 1) *
+                               ((b.n[0] + 63) / 64);
+    const long long warps = 148 * MPLB_LP_MIN_BLOCKS * kSplitWarps;
+    int tasks = 1;
+    while (tasks < kStageTasks && segments > tasks * warps) tasks *= 2;
+    return tasks;
+}
+
 template <int D, typename T>
 cudaError_t Launch<D, T>::StepPart(int part, cudaStream_t s, const BlockDev& b,
                                    const PhysConst& pc, const T* src, T* dst) {
     if (!b.split || (part != 1 && part != 2)) return cudaErrorInvalidValue;
-    const long long blocks = SplitBlocks<D, T>(b);
+    const int tasks = StageTasks<D, T>(b);
+    const long long blocks = SplitBlocks<D, T>(b, tasks);
     if (blocks == 0) return cudaErrorInvalidConfiguration;
     const long long shell = SplitShellBlocks<D>(b);
     // part 1: x faces and interior rows (CTAs shell .. blocks - 1);
@@ -51,10 +77,10 @@ cudaError_t Launch<D, T>::StepPart(int part, cudaStream_t s, const BlockDev& b,
     const int smem = StagedStep<T>() ? StageSmemBytes<D, T>() : 0;
     if (b.off32)
         SplitStepKernel<D, T, true><<<grid, kStepThreads, smem, s>>>(
-            b, pc, src, dst, blk0, 0u);
+            b, pc, src, dst, blk0, 0u, tasks);
     else
         SplitStepKernel<D, T, false><<<grid, kStepThreads, smem, s>>>(
-            b, pc, src, dst, blk0, 0u);
+            b, pc, src, dst, blk0, 0u, tasks);
     return cudaGetLastError();
 }
 
@@ -64,7 +90,7 @@ cudaError_t Launch<D, T>::Step(int mode, dim3 grid, cudaStream_t s,
                                const T* src, T* dst, double* o0, double* o1,
                                double* o2, double* o3) {
     if (mode == kModeStep && b.split) {
-        if (SplitBlocks<D, T>(b) == 0) return cudaErrorInvalidConfiguration;
+        const int tasks = StageTasks<D, T>(b);
         // the shell rows interleaved with the chunks: spc of them after
         // each chunk's CTAs
         const long long nsr = SplitShellBlocks<D>(b);
@@ -72,19 +98,24 @@ cudaError_t Launch<D, T>::Step(int mode, dim3 grid, cudaStream_t s,
             (long long)(b.n[1] - 2) * (D == 3 ? b.n[2] - 2 : 1);
         const long long chunks = (rows + kSplitRows - 1) / kSplitRows;
         const long long per_chunk =
-            SplitChunkCtas<SplitGroup<T>(), StagedStep<T>()>(b.n[0]);
-        const long long spc = (nsr + chunks - 1) / chunks;
-        const long long blocks = chunks * (per_chunk + spc);
+            SplitChunkCtas<SplitGroup<T>(), StagedStep<T>()>(b.n[0], tasks);
+        const long long all = nsr + chunks * per_chunk;
+        const bool walls_first = WallsFirst<T>(b, Lattice<D>::Q);
+        const unsigned spc = walls_first
+                                 ? kWallsFirst
+                                 : (unsigned)((nsr + chunks - 1) / chunks);
+        const long long blocks =
+            walls_first ? all : chunks * (per_chunk + spc);
         if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
         const int smem = StagedStep<T>() ? StageSmemBytes<D, T>() : 0;
         if (b.off32)
             SplitStepKernel<D, T, true><<<(unsigned)blocks, kStepThreads, smem,
-                                          s>>>(b, pc, src, dst, 0u,
-                                               (unsigned)spc);
+                                          s>>>(b, pc, src, dst, 0u, spc,
+                                               tasks);
         else
             SplitStepKernel<D, T, false><<<(unsigned)blocks, kStepThreads,
                                            smem, s>>>(b, pc, src, dst, 0u,
-                                                      (unsigned)spc);
+                                                      spc, tasks);
     } else if (mode == kModeStep && b.off32)
         StepKernel<D, T, kModeStep, true><<<grid, kStepThreads, 0, s>>>(
             b, pc, src, dst, o0, o1, o2, o3);
@@ -198,7 +229,7 @@ cudaError_t Launch<D, T>::HaloFused(cudaStream_t s, const HaloFusedDev& h,
 template <typename T, bool GATHER, bool BC, bool O32>
 cudaError_t LaunchSplitSwap(cudaStream_t s, const BlockDev& b,
                             const PhysConst& pc, T* f) {
-    const long long blocks = SplitBlocks<3, T, false>(b);
+    const long long blocks = SplitBlocks<3, T, false>(b, 1);
     if (blocks == 0) return cudaErrorInvalidConfiguration;
     SplitSwapKernel<T, GATHER, BC, O32><<<(unsigned)blocks, kStepThreads, 0,
                                           s>>>(b, pc, f);

@@ -35,6 +35,7 @@ struct DevBlock {
     void* pop[2] = {nullptr, nullptr};   // form T of the context
     RegionInfo* regions = nullptr;
     RegionOp* ops = nullptr;
+    WallOp* wops = nullptr;              // LOCAL regions' (UploadOps)
     double* stale = nullptr;
     double* fdef = nullptr;
     int* dops_flat = nullptr;
@@ -72,7 +73,12 @@ struct mplbgpu_ctx {
     bool halos_pending = true;
     std::vector<bool> initialised;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // the last step call's device time is ev[ev_end] - ev[ev_start]
+    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    int ev_start = 0, ev_end = 1;
+    // nothing but step calls queued on the stream since ev[ev_end]
+    bool ev_chain = false;
+    bool stream_shared = false;   // mplbgpu_get_stream handed it out
     // a step's independent launches (each block's step, deferred outlets)
     // on side streams forked from `stream` and joined before the halos
     static constexpr int kSides = 3;
@@ -81,7 +87,7 @@ struct mplbgpu_ctx {
     cudaEvent_t join[kSides] = {nullptr, nullptr, nullptr};
     int nlanes = 1;         // streams a step uses (1: no fork)
     float last_ms = 0;
-    bool timing_pending = false;  // ev0/ev1 of the last step call unread
+    bool timing_pending = false;  // the last step call's events unread
     bool begun = false;           // mplbgpu_step_begin without its finish
     long long launches = 0;
     unsigned long long step_count = 0;
@@ -160,6 +166,7 @@ void FreeAll(mplbgpu_ctx* c) {
         cudaFree(b.pop[1]);
         cudaFree(b.regions);
         cudaFree(b.ops);
+        cudaFree(b.wops);
         cudaFree(b.stale);
         cudaFree(b.fdef);
         cudaFree(b.dops_flat);
@@ -187,9 +194,50 @@ void FreeAll(mplbgpu_ctx* c) {
         if (c->join[k]) cudaEventDestroy(c->join[k]);
     }
     if (c->fork) cudaEventDestroy(c->fork);
-    if (c->ev0) cudaEventDestroy(c->ev0);
-    if (c->ev1) cudaEventDestroy(c->ev1);
+    for (cudaEvent_t e : c->ev)
+        if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
+}
+
+// The operations of a block in the order of their indices, and by region in
+// the form the step kernels stage.
+cudaError_t UploadOps(const Plan& P, const BlockPlan& B, DevBlock& b) {
+    std::vector<WallOp> by(kNumRegions * kMaxOps);
+    std::memset(static_cast<void*>(by.data()), 0, by.size() * sizeof(WallOp));
+    const bool f64 = P.precision == MPLBGPU_FP64;
+    for (int r = 0; r < kNumRegions; r++)
+        for (int j = 0; B.region[r].cls >= 0 && j < B.region[r].nops; j++) {
+            const int at = B.region[r].op[j];
+            const RegionOp& op = B.ops[at];
+            WallOp& w = by[r * kMaxOps + j];
+            w.kind = op.kind;
+            w.in = op.in_mask;
+            w.out = op.out_mask;
+            w.par = op.par_mask;
+            w.per_node = op.node_ops != nullptr ? b.ops + at : nullptr;
+            if (f64) {
+                w.denom = op.denom;
+            } else {
+                w.fc[0] = op.c0f;
+                w.fc[1] = op.invf;
+            }
+            for (int i = 0; i < kMaxQ; i++) {
+                const bool par = op.par_mask >> i & 1u;
+                if (f64) {
+                    w.k[i] = par ? op.a[i] : op.b[i];
+                } else {
+                    w.kf[i] = par ? op.af[i] : op.bf[i];
+                    w.am1f[i] = op.am1f[i];
+                }
+            }
+        }
+    cudaError_t e = cudaSuccess;
+    if (!B.ops.empty())
+        e = cudaMemcpy(b.ops, B.ops.data(), B.ops.size() * sizeof(RegionOp),
+                       cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpy(b.wops, by.data(), by.size() * sizeof(WallOp),
+                      cudaMemcpyHostToDevice);
 }
 
 // n doubles set to v (a macroscopic field not given at initialisation).
@@ -208,6 +256,33 @@ cudaError_t FillZeroF(mplbgpu_ctx* c, void* p, long long popstride) {
                                           popstride, Q, c->pc);
     return Launch<3, __half>::FillZero(c->stream, static_cast<__half*>(p),
                                        popstride, Q, c->pc);
+}
+
+// Start and end of a step call's device time.  Step calls that follow one
+// another while the GPU is still on the last one start where it ended, so its
+// end event serves as the next one's start: each timed event holds the stream
+// for about 1.8 us, and a call a step is the reference's way of stepping.
+// Every other entry point waits for the stream or clears ev_chain.
+int TimeStart(mplbgpu_ctx* ctx) {
+    if (ctx->ev_chain && !ctx->stream_shared &&
+        cudaEventQuery(ctx->ev[ctx->ev_end]) == cudaErrorNotReady) {
+        (void)cudaGetLastError();   // not ready is no error
+        ctx->ev_start = ctx->ev_end;
+    } else {
+        ctx->ev_start = (ctx->ev_end + 1) % 3;
+        CK(cudaEventRecord(ctx->ev[ctx->ev_start], ctx->stream));
+    }
+    ctx->ev_end = (ctx->ev_start + 1) % 3;
+    ctx->ev_chain = false;
+    ctx->timing_pending = false;
+    return MPLBGPU_OK;
+}
+
+int TimeEnd(mplbgpu_ctx* ctx) {
+    CK(cudaEventRecord(ctx->ev[ctx->ev_end], ctx->stream));
+    ctx->ev_chain = true;
+    ctx->timing_pending = true;
+    return MPLBGPU_OK;
 }
 
 int EnsureScratch(mplbgpu_ctx* ctx, size_t elems) {
@@ -500,6 +575,7 @@ int FaceSetup(mplbgpu_ctx* ctx, int block, int surface, bool exp,
 template <int D, typename T>
 int FaceCopy(mplbgpu_ctx* ctx, size_t bi, const FaceDev& fd, bool exp,
                     void* buf) {
+    ctx->ev_chain = false;
     DevBlock& b = ctx->blocks[bi];
     const long long total = (long long)fd.npop * fd.nu * fd.nv;
     const unsigned grid =
@@ -570,9 +646,9 @@ mplbgpu_status mplbgpu_create(const mplbgpu_desc* desc, mplbgpu_ctx** out) {
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) !=
         cudaSuccess)
         return fail_cuda(e, "cudaStreamCreate");
-    if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess ||
-        (e = cudaEventCreate(&c->ev1)) != cudaSuccess)
-        return fail_cuda(e, "cudaEventCreate");
+    for (cudaEvent_t& ev : c->ev)
+        if ((e = cudaEventCreate(&ev)) != cudaSuccess)
+            return fail_cuda(e, "cudaEventCreate");
     {
         // independent launches per step: every block's step kernel and
         // every block's deferred kernels (two-array scheme)
@@ -620,13 +696,13 @@ mplbgpu_status mplbgpu_create(const mplbgpu_desc* desc, mplbgpu_ctx** out) {
             (e = cudaMemcpy(b.regions, B.region, sizeof(B.region),
                             cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail_cuda(e, "region table");
-        if (!B.ops.empty()) {
-            const size_t ob = B.ops.size() * sizeof(RegionOp);
-            if ((e = cudaMalloc(&b.ops, ob)) != cudaSuccess ||
-                (e = cudaMemcpy(b.ops, B.ops.data(), ob,
-                                cudaMemcpyHostToDevice)) != cudaSuccess)
-                return fail_cuda(e, "op table");
-        }
+        if ((!B.ops.empty() &&
+             (e = cudaMalloc(&b.ops, B.ops.size() * sizeof(RegionOp))) !=
+                 cudaSuccess) ||
+            (e = cudaMalloc(&b.wops, kNumRegions * kMaxOps *
+                                         sizeof(WallOp))) != cudaSuccess ||
+            (e = UploadOps(P, B, b)) != cudaSuccess)
+            return fail_cuda(e, "op table");
         if (B.nstale > 0 &&
             (e = cudaMalloc(&b.stale, (size_t)B.nstale * Q * sizeof(double))) !=
                 cudaSuccess)
@@ -690,6 +766,7 @@ mplbgpu_status mplbgpu_create(const mplbgpu_desc* desc, mplbgpu_ctx** out) {
         d.popstride = B.popstride;
         d.regions = b.regions;
         d.ops = b.ops;
+        d.wops = b.wops;
         d.stale = b.stale;
         d.fdef = b.fdef;
         d.ndef = B.ndeferred;
@@ -733,6 +810,8 @@ mplbgpu_status mplbgpu_create(const mplbgpu_desc* desc, mplbgpu_ctx** out) {
             const RegionInfo& R = B.region[r];
             d.rflags[r] = (uint8_t)((R.cls < 0 ? kPure : R.cls) |
                                     (R.fluidlike ? 4 : 0));
+            d.rnops[r] = (uint8_t)(R.cls < 0 ? 0 : R.nops);
+            d.rside[r] = (int)R.side_base;
             d.rpull[r] = R.pull;
             d.rstale[r] = R.stale;
         }
@@ -956,16 +1035,15 @@ mplbgpu_status mplbgpu_step(mplbgpu_ctx* ctx, int nsteps) {
         rc = RunHalos(ctx);
         if (rc != MPLBGPU_OK) return rc;
     }
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
+    rc = TimeStart(ctx);
+    if (rc != MPLBGPU_OK) return rc;
     for (int s = 0; s < nsteps; s++) {
         rc = MPLB_DISPATCH(ctx, StepOnce, ctx);
         if (rc != MPLBGPU_OK) return rc;
     }
     // no host wait: the caller's next reading call (download, residual,
     // mass, synchronize, last_step_ms) waits for the stream
-    CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    ctx->timing_pending = true;
-    return MPLBGPU_OK;
+    return TimeEnd(ctx);
 }
 
 mplbgpu_status mplbgpu_step_begin(mplbgpu_ctx* ctx) {
@@ -979,7 +1057,8 @@ mplbgpu_status mplbgpu_step_begin(mplbgpu_ctx* ctx) {
         rc = RunHalos(ctx);
         if (rc != MPLBGPU_OK) return rc;
     }
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
+    rc = TimeStart(ctx);
+    if (rc != MPLBGPU_OK) return rc;
     return StepBegin(ctx);
 }
 
@@ -990,13 +1069,12 @@ mplbgpu_status mplbgpu_step_finish(mplbgpu_ctx* ctx) {
                       "mplbgpu_step_finish without mplbgpu_step_begin");
     int rc = StepFinish(ctx);
     if (rc != MPLBGPU_OK) return rc;
-    CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    ctx->timing_pending = true;
-    return MPLBGPU_OK;
+    return TimeEnd(ctx);
 }
 
 mplbgpu_status mplbgpu_get_stream(mplbgpu_ctx* ctx, void** stream) {
     if (!ctx || !stream) return MPLBGPU_ERR_INVALID;
+    ctx->stream_shared = true;   // the caller may queue work of its own
     *stream = static_cast<void*>(ctx->stream);
     return MPLBGPU_OK;
 }
@@ -1269,8 +1347,7 @@ mplbgpu_status mplbgpu_set_boundary_velocity(mplbgpu_ctx* ctx, int boundary,
             op.fext[a] = ext[a];
         }
     }
-    CK(cudaMemcpy(b.ops, B.ops.data(), B.ops.size() * sizeof(RegionOp),
-                  cudaMemcpyHostToDevice));
+    CK(UploadOps(ctx->plan, B, b));
     return MPLBGPU_OK;
 }
 
@@ -1294,8 +1371,9 @@ long long mplbgpu_launch_count(const mplbgpu_ctx* ctx) {
 mplbgpu_status mplbgpu_last_step_ms(mplbgpu_ctx* ctx, float* ms) {
     if (!ctx || !ms) return MPLBGPU_ERR_INVALID;
     if (ctx->timing_pending) {
-        CK(cudaEventSynchronize(ctx->ev1));
-        CK(cudaEventElapsedTime(&ctx->last_ms, ctx->ev0, ctx->ev1));
+        CK(cudaEventSynchronize(ctx->ev[ctx->ev_end]));
+        CK(cudaEventElapsedTime(&ctx->last_ms, ctx->ev[ctx->ev_start],
+                                ctx->ev[ctx->ev_end]));
         ctx->timing_pending = false;
     }
     *ms = ctx->last_ms;

@@ -41,15 +41,24 @@ enum OpKind : int { kOpEqm = 1, kOpHbb = 2, kOpExtrapol = 3, kOpZero = 4 };
 // One boundary operation specialised to one region's geometry.  All FP64
 // constants that depend only on the boundary's given values are computed
 // here in the reference's operation order.
-struct RegionOp {
+// The first 16 bytes (the head) and the 16 after them are what a kernel needs
+// before the arrays.
+struct alignas(16) RegionOp {
     int kind;
-    int bc;             // index of the boundary (definition order)
     uint32_t in_mask;   // EQM: incoming;  EXTRAPOL: copied populations
     uint32_t out_mask;  // EQM: outgoing;  HBB: bounced populations
     uint32_t par_mask;  // EQM: parallel
+    double denom;       // EQM: (1 - deltaRho) - rhoParallel
+    // EQM / HBB with a wall velocity per node (mplbgpu_set_boundary_velocity):
+    // this operation evaluated for every node of the boundary's surface
+    // range (x fastest, from node forg) with that node's velocity; null:
+    // the constants here (uniform given values) hold for every node
+    const RegionOp* node_ops;
+    int bc;             // index of the boundary (definition order)
     int nb_axis;        // EXTRAPOL copy source axis (-1: none)
     int nb_sign;
-    double denom;       // EQM: (1 - deltaRho) - rhoParallel
+    int forg[3];
+    int fext[3];
     double win;         // EQM: sum of the incoming weights (shifted forms)
     double c0;          // EQM: 2 win - denom, so rhoWall - 1 =
                         //      (c0 + 2 sum_in h) / denom (shifted forms)
@@ -61,13 +70,6 @@ struct RegionOp {
     // arrays above rounded to float (SetFloatConsts)
     float invf, c0f;
     float am1f[kMaxQ], af[kMaxQ], bf[kMaxQ];
-    // EQM / HBB with a wall velocity per node (mplbgpu_set_boundary_velocity):
-    // this operation evaluated for every node of the boundary's surface
-    // range (x fastest, from node forg) with that node's velocity; null:
-    // the constants above (uniform given values) hold for every node
-    const RegionOp* node_ops;
-    int forg[3];
-    int fext[3];
 };
 
 struct RegionInfo {

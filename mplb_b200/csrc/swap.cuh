@@ -50,7 +50,8 @@ __device__ __forceinline__ void SwapNode(const BlockDev& b,
                                          double* __restrict__ out1,
                                          double* __restrict__ out2,
                                          double* __restrict__ out3, int x,
-                                         int y, int z) {
+                                         int y, int z, bool valid,
+                                         const WallOp* ops, bool staged) {
     using L = Lattice<3>;
     using P = Prec<T>;
     using C = typename P::C;
@@ -62,14 +63,20 @@ __device__ __forceinline__ void SwapNode(const BlockDev& b,
     // opposite map, and it has no boundary programme
     const uint32_t exch = GATHER ? (interior ? ~1u : b.swap_exch[r]) : 0u;
     C v[Q];
+    if (valid) {
 #pragma unroll
-    for (int k = 0; k < Q; k++)
-        v[k] = P::Load(f, SwapSlot<O32>(b, node, k, exch >> k & 1u), k, pc);
-    if (BC && !interior) {
-        const RegionInfo& R = b.regions[r];
-        for (int i = 0; i < R.nops; i++)
-            ApplyEqm<L, T>(v, b.ops[R.op[i]], pc, x, y, z);
+        for (int k = 0; k < Q; k++)
+            v[k] = P::Load(f, SwapSlot<O32>(b, node, k, exch >> k & 1u), k,
+                           pc);
     }
+    if (staged) {
+        CpAsyncWait<0>();
+        __syncthreads();
+    }
+    if (!valid) return;
+    if (BC && !interior)
+        ApplyWallOps<L, T>(v, ops + (r % 3) * kMaxOps, b.rnops[r], pc, f, b,
+                           node, x, y, z);
     const bool fl = (b.rflags[r] & 4) != 0;
     if (MODE == kModeF) {
         const long long dn =
@@ -119,10 +126,14 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
     SwapKernel(BlockDev b, PhysConst pc, T* f, double* __restrict__ out0,
                double* __restrict__ out1, double* __restrict__ out2,
                double* __restrict__ out3) {
+    __shared__ WallOp ops[kRowOps];
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= b.n[0]) return;
-    SwapNode<T, MODE, GATHER, BC, O32>(b, pc, f, out0, out1, out2, out3, x,
-                                       blockIdx.y, blockIdx.z);
+    const int rb = RegionOf(0, blockIdx.y, blockIdx.z, b.n, 3);
+    const bool staged = BC && RowHasOps(b, rb, blockIdx.x * blockDim.x);
+    if (staged) StageWallOps(b, rb, ops);
+    SwapNode<T, MODE, GATHER, BC, O32>(b, pc, f, out0, out1, out2, out3,
+                                       min(x, b.n[0] - 1), blockIdx.y,
+                                       blockIdx.z, x < b.n[0], ops, staged);
 }
 
 // The G interior nodes x0 + 32 j of one row (the layout of
@@ -195,6 +206,7 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
                                            ? MPLB_SWAP_F64_MIN_BLOCKS
                                            : MPLB_LP_MIN_BLOCKS)
     SplitSwapKernel(BlockDev b, PhysConst pc, T* f) {
+    __shared__ WallOp ops[kRowOps];
     const int nbx = (b.n[0] + (int)blockDim.x - 1) / (int)blockDim.x;
     const int ny = b.n[1] - 2;
     const int nz = b.n[2];
@@ -202,8 +214,8 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
     unsigned blk = blockIdx.x;
     if (blk < nsr) {
         const int row = (int)(blk / nbx);
-        const int x = (int)(blk % nbx) * blockDim.x + threadIdx.x;
-        if (x >= b.n[0]) return;
+        const int x0 = (int)(blk % nbx) * blockDim.x;
+        const int x = x0 + threadIdx.x;
         int y, z;
         if (row < 2 * nz) {
             y = (row & 1) ? b.n[1] - 1 : 0;
@@ -213,8 +225,12 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
             z = (r2 & 1) ? b.n[2] - 1 : 0;
             y = 1 + (r2 >> 1);
         }
-        SwapNode<T, kModeStep, GATHER, BC, O32>(b, pc, f, nullptr, nullptr,
-                                                nullptr, nullptr, x, y, z);
+        const int rb = RegionOf(0, y, z, b.n, 3);
+        const bool staged = BC && RowHasOps(b, rb, x0);
+        if (staged) StageWallOps(b, rb, ops);
+        SwapNode<T, kModeStep, GATHER, BC, O32>(
+            b, pc, f, nullptr, nullptr, nullptr, nullptr,
+            min(x, b.n[0] - 1), y, z, x < b.n[0], ops, staged);
         return;
     }
     blk -= nsr;
@@ -224,12 +240,15 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
     const int chunk = (int)(blk / per_chunk);
     const int w = (int)(blk % per_chunk);
     if (w == 0) {
-        const int r = chunk * kSplitRows + (int)(threadIdx.x >> 1);
-        if (threadIdx.x >= 2 * kSplitRows || r >= rows) return;
+        const int t = chunk * kSplitRows + (int)(threadIdx.x >> 1);
+        const int r = min(t, rows - 1);
         const int x = (threadIdx.x & 1) ? b.n[0] - 1 : 0;
-        SwapNode<T, kModeStep, GATHER, BC, O32>(b, pc, f, nullptr, nullptr,
-                                                nullptr, nullptr, x,
-                                                1 + r % ny, 1 + r / ny);
+        constexpr int rb = 12;   // interior rows: the x faces are 12 and 14
+        const bool staged = BC && (b.rnops[rb] | b.rnops[rb + 2]) != 0;
+        if (staged) StageWallOps(b, rb, ops);
+        SwapNode<T, kModeStep, GATHER, BC, O32>(
+            b, pc, f, nullptr, nullptr, nullptr, nullptr, x, 1 + r % ny,
+            1 + r / ny, t < rows, ops, staged);
         return;
     }
     const SplitTask k = InteriorTask<G>(b, chunk, w);
