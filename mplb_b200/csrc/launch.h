@@ -12,7 +12,9 @@ namespace mplb {
 
 template <int D, typename T>
 struct Launch {
-    static cudaError_t Step(int mode, dim3 grid, cudaStream_t s,
+    // `over` (here and below): a kernel of a step that may start over the
+    // tail of the one queued before it on the stream, itself one of these
+    static cudaError_t Step(int mode, bool over, dim3 grid, cudaStream_t s,
                             const BlockDev& b, const PhysConst& pc,
                             const T* src, T* dst, double* o0, double* o1,
                             double* o2, double* o3);
@@ -47,8 +49,9 @@ struct Launch {
                                      const T* fdirect, double* o0, double* o1,
                                      double* o2, double* o3);
     // every halo copy of a step in one launch (pop[cur] is current)
-    static cudaError_t HaloFused(cudaStream_t s, const HaloFusedDev& h,
-                                 int cur, unsigned ctas);
+    static cudaError_t HaloFused(bool over, cudaStream_t s,
+                                 const HaloFusedDev& h, int cur,
+                                 unsigned ctas);
     // face exchange of a decomposed block: export (block -> buf) or import
     static cudaError_t Face(bool exp, unsigned grid, cudaStream_t s,
                             const BlockDev& b, const FaceDev& fd, T* f,
@@ -56,7 +59,8 @@ struct Launch {
     // swap scheme (3D only): one step (kModeStep) or an observation of the
     // current f, from the array in place; gather: slots at their streamed
     // places; bc: boundary programme pending
-    static cudaError_t Swap(int mode, bool gather, bool bc, dim3 grid,
+    static cudaError_t Swap(int mode, bool over, bool gather, bool bc,
+                            dim3 grid,
                             cudaStream_t s, const BlockDev& b,
                             const PhysConst& pc, T* f, double* o0, double* o1,
                             double* o2, double* o3);

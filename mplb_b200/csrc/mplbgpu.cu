@@ -33,9 +33,11 @@ thread_local std::string g_create_error;
 struct DevBlock {
     BlockDev dev{};
     void* pop[2] = {nullptr, nullptr};   // form T of the context
+    // one allocation: region records, LOCAL regions' operations as the step
+    // kernels stage them, all operations
     RegionInfo* regions = nullptr;
+    WallOp* wops = nullptr;
     RegionOp* ops = nullptr;
-    WallOp* wops = nullptr;              // LOCAL regions' (UploadOps)
     double* stale = nullptr;
     double* fdef = nullptr;
     int* dops_flat = nullptr;
@@ -165,8 +167,6 @@ void FreeAll(mplbgpu_ctx* c) {
         cudaFree(b.pop[0]);
         cudaFree(b.pop[1]);
         cudaFree(b.regions);
-        cudaFree(b.ops);
-        cudaFree(b.wops);
         cudaFree(b.stale);
         cudaFree(b.fdef);
         cudaFree(b.dops_flat);
@@ -231,12 +231,13 @@ cudaError_t UploadOps(const Plan& P, const BlockPlan& B, DevBlock& b) {
                 }
             }
         }
-    cudaError_t e = cudaSuccess;
+    // the two tables follow each other
+    const size_t wbytes = by.size() * sizeof(WallOp);
+    std::vector<char> both(wbytes + B.ops.size() * sizeof(RegionOp));
+    std::memcpy(both.data(), by.data(), wbytes);
     if (!B.ops.empty())
-        e = cudaMemcpy(b.ops, B.ops.data(), B.ops.size() * sizeof(RegionOp),
-                       cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpy(b.wops, by.data(), by.size() * sizeof(WallOp),
+        std::memcpy(both.data() + wbytes, B.ops.data(), both.size() - wbytes);
+    return cudaMemcpy(b.wops, both.data(), both.size(),
                       cudaMemcpyHostToDevice);
 }
 
@@ -298,26 +299,28 @@ int EnsureScratch(mplbgpu_ctx* ctx, size_t elems) {
 // Every halo copy of the step (Field::TransferHalos in CreateHalos order)
 // in one launch.
 template <int D, typename T>
-int RunHalosT(mplbgpu_ctx* ctx) {
+int RunHalosT(mplbgpu_ctx* ctx, bool over) {
     if (!ctx->halos.empty())
-        CK_LAUNCH_E(Launch<D, T>::HaloFused(ctx->stream, ctx->hfd, ctx->cur,
-                                            ctx->halo_ctas));
+        CK_LAUNCH_E(Launch<D, T>::HaloFused(over, ctx->stream, ctx->hfd,
+                                            ctx->cur, ctx->halo_ctas));
     ctx->halos_pending = false;
     return MPLBGPU_OK;
 }
 
-int RunHalos(mplbgpu_ctx* ctx) { return MPLB_DISPATCH(ctx, RunHalosT, ctx); }
+int RunHalos(mplbgpu_ctx* ctx) {
+    return MPLB_DISPATCH(ctx, RunHalosT, ctx, false);
+}
 
 // One step of the swap scheme (single block, no halos): from f itself or
 // the streamed state the node reads its own slots, from the locally swapped
 // state it gathers the streamed slots.
 template <int D, typename T>
-int SwapStepOnce(mplbgpu_ctx* ctx) {
+int SwapStepOnce(mplbgpu_ctx* ctx, bool over) {
     ctx->pc.seed = (uint32_t)(++ctx->step_count);
     DevBlock& b = ctx->blocks[0];
     const BlockPlan& B = ctx->plan.blocks[0];
     const int st = ctx->swap_state;
-    CK_LAUNCH_E(Launch<D, T>::Swap(kModeStep, st == 1, st != 0,
+    CK_LAUNCH_E(Launch<D, T>::Swap(kModeStep, over, st == 1, st != 0,
                                    NodeGrid(B, D), ctx->stream, b.dev, ctx->pc,
                                    static_cast<T*>(b.pop[0]), nullptr, nullptr,
                                    nullptr, nullptr));
@@ -331,10 +334,12 @@ int SwapStepOnce(mplbgpu_ctx* ctx) {
 // previous array and write disjoint nodes of the new one - go round-robin
 // over the context's stream and its side streams (forked after the previous
 // step's halos, joined before this step's), so that one launch's tail
-// overlaps the next one's start.
+// overlaps the next one's start.  A step on one stream that follows another of
+// the same call (`over`) starts over that one's tail, and its halos over its
+// own.
 template <int D, typename T>
-int StepOnce(mplbgpu_ctx* ctx) {
-    if (ctx->plan.swap) return SwapStepOnce<D, T>(ctx);
+int StepOnce(mplbgpu_ctx* ctx, bool over) {
+    if (ctx->plan.swap) return SwapStepOnce<D, T>(ctx, over);
     const int src = ctx->cur, dst = 1 - ctx->cur;
     ctx->pc.seed = (uint32_t)(++ctx->step_count);
     const int lanes = ctx->nlanes;
@@ -354,8 +359,8 @@ int StepOnce(mplbgpu_ctx* ctx) {
         const BlockPlan& B = ctx->plan.blocks[bi];
         const T* s = static_cast<const T*>(b.pop[src]);
         T* d = static_cast<T*>(b.pop[dst]);
-        CK_LAUNCH_E(Launch<D, T>::Step(kModeStep, NodeGrid(B, D), next(),
-                                       b.dev, ctx->pc, s, d, nullptr, nullptr,
+        CK_LAUNCH_E(Launch<D, T>::Step(kModeStep, over && lanes == 1,
+                                       NodeGrid(B, D), next(), b.dev, ctx->pc, s, d, nullptr, nullptr,
                                        nullptr, nullptr));
         if (B.ndeferred > 0 && b.dev.deferred_fused) {
             const unsigned g = (unsigned)((B.ndeferred + kThreads - 1) / kThreads);
@@ -387,7 +392,7 @@ int StepOnce(mplbgpu_ctx* ctx) {
     }
     ctx->cur = dst;
     ctx->initial = false;
-    return RunHalosT<D, T>(ctx);
+    return RunHalosT<D, T>(ctx, lanes == 1);
 }
 
 // First part of a step: the x faces and interior rows of every block with
@@ -422,7 +427,7 @@ int StepFinishT(mplbgpu_ctx* ctx) {
             CK_LAUNCH_E(Launch<D, T>::StepPart(2, ctx->stream, b.dev, ctx->pc,
                                                s, d));
         } else {
-            CK_LAUNCH_E(Launch<D, T>::Step(kModeStep, NodeGrid(B, D),
+            CK_LAUNCH_E(Launch<D, T>::Step(kModeStep, false, NodeGrid(B, D),
                                            ctx->stream, b.dev, ctx->pc, s, d,
                                            nullptr, nullptr, nullptr,
                                            nullptr));
@@ -450,7 +455,7 @@ int StepFinishT(mplbgpu_ctx* ctx) {
     ctx->cur = dst;
     ctx->initial = false;
     ctx->begun = false;
-    return RunHalosT<D, T>(ctx);
+    return RunHalosT<D, T>(ctx, false);
 }
 
 int StepBegin(mplbgpu_ctx* ctx) { return MPLB_DISPATCH(ctx, StepBeginT, ctx); }
@@ -466,7 +471,7 @@ int Observe(mplbgpu_ctx* ctx, int mode, size_t bi, double* o0, double* o1,
     const BlockPlan& B = ctx->plan.blocks[bi];
     if (ctx->plan.swap) {
         const int st = ctx->swap_state;
-        CK_LAUNCH_E(Launch<D, T>::Swap(mode, st == 1, st != 0, NodeGrid(B, D),
+        CK_LAUNCH_E(Launch<D, T>::Swap(mode, false, st == 1, st != 0, NodeGrid(B, D),
                                        ctx->stream, b.dev, ctx->pc,
                                        static_cast<T*>(b.pop[0]), o0, o1, o2,
                                        o3));
@@ -480,7 +485,7 @@ int Observe(mplbgpu_ctx* ctx, int mode, size_t bi, double* o0, double* o1,
                                                 pv, o0, o1, o2, o3));
         return MPLBGPU_OK;
     }
-    CK_LAUNCH_E(Launch<D, T>::Step(mode, NodeGrid(B, D), ctx->stream, b.dev,
+    CK_LAUNCH_E(Launch<D, T>::Step(mode, false, NodeGrid(B, D), ctx->stream, b.dev,
                                    ctx->pc, pv, nullptr, o0, o1, o2, o3));
     if (B.ndeferred > 0) {
         const unsigned g = (unsigned)((B.ndeferred + kThreads - 1) / kThreads);
@@ -692,16 +697,21 @@ mplbgpu_status mplbgpu_create(const mplbgpu_desc* desc, mplbgpu_ctx** out) {
                                     0, slack, c->stream);
             if (e != cudaSuccess) return fail_cuda(e, "population fill");
         }
-        if ((e = cudaMalloc(&b.regions, sizeof(B.region))) != cudaSuccess ||
+        const size_t rbytes = (sizeof(B.region) + 255) / 256 * 256;
+        const size_t wbytes = kNumRegions * kMaxOps * sizeof(WallOp);
+        static_assert(sizeof(WallOp) * kMaxOps % 16 == 0, "aligned tables");
+        if ((e = cudaMalloc(&b.regions,
+                            rbytes + wbytes +
+                                B.ops.size() * sizeof(RegionOp))) !=
+                cudaSuccess ||
             (e = cudaMemcpy(b.regions, B.region, sizeof(B.region),
                             cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail_cuda(e, "region table");
-        if ((!B.ops.empty() &&
-             (e = cudaMalloc(&b.ops, B.ops.size() * sizeof(RegionOp))) !=
-                 cudaSuccess) ||
-            (e = cudaMalloc(&b.wops, kNumRegions * kMaxOps *
-                                         sizeof(WallOp))) != cudaSuccess ||
-            (e = UploadOps(P, B, b)) != cudaSuccess)
+        b.wops = reinterpret_cast<WallOp*>(
+            reinterpret_cast<char*>(b.regions) + rbytes);
+        b.ops = reinterpret_cast<RegionOp*>(
+            reinterpret_cast<char*>(b.wops) + wbytes);
+        if ((e = UploadOps(P, B, b)) != cudaSuccess)
             return fail_cuda(e, "op table");
         if (B.nstale > 0 &&
             (e = cudaMalloc(&b.stale, (size_t)B.nstale * Q * sizeof(double))) !=
@@ -1038,7 +1048,7 @@ mplbgpu_status mplbgpu_step(mplbgpu_ctx* ctx, int nsteps) {
     rc = TimeStart(ctx);
     if (rc != MPLBGPU_OK) return rc;
     for (int s = 0; s < nsteps; s++) {
-        rc = MPLB_DISPATCH(ctx, StepOnce, ctx);
+        rc = MPLB_DISPATCH(ctx, StepOnce, ctx, s > 0);
         if (rc != MPLBGPU_OK) return rc;
     }
     // no host wait: the caller's next reading call (download, residual,

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
                double* __restrict__ out1, double* __restrict__ out2,
                double* __restrict__ out3) {
     __shared__ WallOp ops[kRowOps];
+    WaitForPrevious();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int rb = RegionOf(0, blockIdx.y, blockIdx.z, b.n, 3);
     const bool staged = BC && RowHasOps(b, rb, blockIdx.x * blockDim.x);
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
                                            : MPLB_LP_MIN_BLOCKS)
     SplitSwapKernel(BlockDev b, PhysConst pc, T* f) {
     __shared__ WallOp ops[kRowOps];
+    WaitForPrevious();
     const int nbx = (b.n[0] + (int)blockDim.x - 1) / (int)blockDim.x;
     const int ny = b.n[1] - 2;
     const int nz = b.n[2];
