@@ -25,6 +25,7 @@ SOURCES = [os.path.join(CSRC, u) for u, _ in UNITS]
 HEADERS = [os.path.join(CSRC, h) for h in ("kernels.cuh", "lattice.h",
                                             "plan.h", "launch.h",
                                             "launch_impl.cuh", "swap.cuh",
+                                            "double_step.cuh",
                                             "batch_kernels.cuh",
                                             "batch_resident.cuh", "tma.cuh",
                                             "nn/umma.cuh", "nn/conv.cuh",

@@ -804,14 +804,13 @@ __device__ __forceinline__ bool RowHasOps(const BlockDev& b, int rb, int x0) {
            (x1 == b.n[0] && b.rnops[rb + 2] != 0);
 }
 
-// The programme of one LOCAL node from its staged operations.
-template <typename L, typename T>
+// The programme of one LOCAL node from its staged operations; own(i):
+// population i of the node itself, before streaming (halfway bounce-back).
+template <typename L, typename T, typename Own>
 __device__ __forceinline__ void ApplyWallOps(typename Prec<T>::C* f,
                                              const WallOp* ops, int nops,
-                                             const PhysConst& pc,
-                                             const T* __restrict__ src,
-                                             const BlockDev& b, long long node,
-                                             int x, int y, int z) {
+                                             const PhysConst& pc, int x, int y,
+                                             int z, Own own) {
     using P = Prec<T>;
     using C = typename P::C;
     constexpr int Q = L::Q;
@@ -829,16 +828,17 @@ __device__ __forceinline__ void ApplyWallOps(typename Prec<T>::C* f,
                               op.fc[1], pc, k,
                               [&](int i) { return op.am1f[i]; });
         } else if (op.kind == kOpHbb) {
-            if (op.per_node != nullptr) {
-                ApplyHbb<L, T>(f, *op.per_node, pc, src, b, node, x, y, z);
-            } else {
-                const uint32_t out = op.out;
+            const RegionOp* node =
+                op.per_node != nullptr ? &NodeOp(*op.per_node, x, y, z)
+                                       : nullptr;
+            const uint32_t out = op.out;
 #pragma unroll
-                for (int i = 0; i < Q; i++)
-                    if (out >> i & 1u)
-                        f[i] = P::Load(src, L::opp(i) * b.popstride + node,
-                                       L::opp(i), pc) + k(i);
-            }
+            for (int i = 0; i < Q; i++)
+                if (out >> i & 1u)
+                    f[i] = own(L::opp(i)) +
+                           (node == nullptr  ? k(i)
+                            : P::kShifted ? (C)node->bf[i]
+                                          : (C)node->b[i]);
         } else if (op.kind == kOpZero) {
             ApplyZero<L, T>(f, pc);
         }
@@ -934,8 +934,11 @@ __device__ __forceinline__ void StepNode(const BlockDev& b,
     }
     if (!valid) return;
     if (cls != kPure)
-        ApplyWallOps<L, T>(f, ops + (r % 3) * kMaxOps, b.rnops[r], pc, src, b,
-                           node, x, y, z);
+        ApplyWallOps<L, T>(f, ops + (r % 3) * kMaxOps, b.rnops[r], pc, x, y, z,
+                           [&](int i) {
+                               return P::Load(src, i * b.popstride + node, i,
+                                              pc);
+                           });
     const bool fl = (rf & 4) != 0;
     if (MODE == kModeF) {
         const long long dn =

@@ -18,6 +18,10 @@ struct Launch {
                             const BlockDev& b, const PhysConst& pc,
                             const T* src, T* dst, double* o0, double* o1,
                             double* o2, double* o3);
+    // two steps of a 2D block in FP64 or FP32 (double_step.cuh)
+    static cudaError_t TwoSteps(bool over, cudaStream_t s, const BlockDev& b,
+                                const PhysConst& pc, const T* src, T* dst,
+                                int periodic);
     // the two parts of a split step (b.split): 1 = the x faces and the
     // interior rows (no node of theirs reads a halo layer beyond a y or z
     // face), 2 = the shell rows
@@ -67,5 +71,8 @@ struct Launch {
 };
 
 constexpr int kStepThreads = 128;
+
+// Population arrays that stay in the L2 cache (126 MB) from step to step.
+constexpr double kL2Bytes = 100e6;
 
 }  // namespace mplb

@@ -2,6 +2,7 @@
 // translation units that instantiate them).
 #pragma once
 
+#include "double_step.cuh"
 #include "launch.h"
 #include "swap.cuh"
 
@@ -64,7 +65,7 @@ cudaError_t LaunchOver(bool over, void (*kernel)(P...), dim3 grid,
 // and written twice in HBM (128^3 in FP64 140 us against 114).
 template <typename T>
 bool WallsFirst(const BlockDev& b, int q) {
-    return 2.0 * q * (double)b.popstride * sizeof(T) <= 100e6;
+    return 2.0 * q * (double)b.popstride * sizeof(T) <= kL2Bytes;
 }
 
 // Row segments a warp of the staged interior takes one after the other: up to
@@ -148,6 +149,25 @@ cudaError_t Launch<D, T>::Step(int mode, bool over, dim3 grid, cudaStream_t s,
         StepKernel<D, T, kModeF><<<grid, kStepThreads, 0, s>>>(
             b, pc, src, dst, o0, o1, o2, o3);
     return cudaGetLastError();
+}
+
+template <int D, typename T>
+cudaError_t Launch<D, T>::TwoSteps(bool over, cudaStream_t s,
+                                   const BlockDev& b, const PhysConst& pc,
+                                   const T* src, T* dst, int periodic) {
+    if constexpr (D != 2 || std::is_same<T, __half>::value) {
+        return cudaErrorInvalidValue;
+    } else {
+        constexpr int kSmem = DoubleSmemBytes<T>();
+        const cudaError_t e = cudaFuncSetAttribute(
+            DoubleStepKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            kSmem);
+        if (e != cudaSuccess) return e;
+        const dim3 grid((b.n[0] + TileW<T>() - 1) / TileW<T>(),
+                        (b.n[1] + kTileH - 1) / kTileH);
+        return LaunchOver(over, DoubleStepKernel<T>, grid, kDoubleThreads,
+                          kSmem, s, b, pc, src, dst, periodic);
+    }
 }
 
 template <int D, typename T>

@@ -75,8 +75,8 @@ __device__ __forceinline__ void SwapNode(const BlockDev& b,
     }
     if (!valid) return;
     if (BC && !interior)
-        ApplyWallOps<L, T>(v, ops + (r % 3) * kMaxOps, b.rnops[r], pc, f, b,
-                           node, x, y, z);
+        ApplyWallOps<L, T>(v, ops + (r % 3) * kMaxOps, b.rnops[r], pc, x, y, z,
+                           [&](int i) { return v[i]; });   // EQM only
     const bool fl = (b.rflags[r] & 4) != 0;
     if (MODE == kModeF) {
         const long long dn =
