@@ -631,6 +631,168 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     }
 }
 
+// The weight gradient of a 3x3 convolution (see conv.cuh): one 32-channel slice
+// of the input, bn output channels, a range of bands of image rows.  Cold-cache
+// layer times (32 images), tap by tap in brackets: 96 -> 32 at 128^2 64 us (202),
+// 32 -> 32 30 (77), 192 -> 64 at 64^2 49 (116), 384 -> 128 at 32^2 51 (78), 128 ->
+// 128 28 (43).  Row by row a sum has as many terms as a tap's: over surplus columns, too,
+// 256 -> 256 at 16^2 rounds 18/16 times as often, 3.0e-7 off the 64-bit sums in
+// place of 2.9e-7.  Rows under 16 pixels, which no layer of the network has, go over
+// them all the same: there a zero of dY meets a pixel of X that the tap does not use.
+__global__ void __launch_bounds__(kConvThreads, 1)
+    WgradBandKernel(const __grid_constant__ CUtensorMap tx,
+                    const __grid_constant__ CUtensorMap tdy,
+                    WgradBandArgs a) {
+    constexpr uint32_t SW = 64;   // bytes of a position: 32 channels
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = Align1024(smem_raw);
+    const int slices = a.bn / 32;
+    const uint32_t stage_bytes = a.x_bytes + slices * a.dy_bytes;
+    uint64_t* full =
+        reinterpret_cast<uint64_t*>(smem + a.stages * stage_bytes);
+    uint64_t* empty = full + a.stages;
+    uint64_t* accum = empty + a.stages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+    volatile int* cta_err = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = 32 * blockIdx.y, n0 = a.bn * blockIdx.z;
+    const int b0 = blockIdx.x * a.bands_per_cta;
+    const int nb = min(a.bands_total, b0 + a.bands_per_cta) - b0;
+    if (nb <= 0) return;   // uniform over the CTA, before any allocation
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.stages; s++) {
+            BarInit(&full[s], 1);
+            BarInit(&empty[s], 1);
+        }
+        BarInit(accum, 1);
+        *cta_err = 0;
+        FenceBarrierInit();
+        PrefetchTmap(&tx);
+        PrefetchTmap(&tdy);
+    }
+    if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    // the positions past a band's last row, which no copy writes, are zero:
+    // they fill up the last 16 positions of the sum
+    for (int s = 0; s < a.stages; s++)
+        for (int i = 0; i <= slices; i++) {
+            uint8_t* at = smem + s * stage_bytes +
+                          (i == 0 ? 0 : a.x_bytes + (i - 1) * a.dy_bytes);
+            const int from = (int)(i == 0 ? a.x_box : a.dy_box) / 16;
+            const int to = (i == 0 ? a.x_bytes : a.dy_bytes) / 16;
+            for (int e = from + (int)threadIdx.x; e < to; e += kConvThreads)
+                reinterpret_cast<uint4*>(at)[e] = make_uint4(0, 0, 0, 0);
+        }
+    FenceProxyAsync();
+    FenceBeforeSync();
+    __syncthreads();
+    FenceAfterSync();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        int j = 0;
+        for (; j < nb; j++) {
+            const int s = j % a.stages;
+            if (j >= a.stages &&
+                !BarWait(&empty[s], ((j / a.stages) + 1) & 1, cta_err)) {
+                Flag(cta_err, a.err);
+                break;
+            }
+            const int img = (b0 + j) / a.bands_per_img;
+            const int r0 = (b0 + j - img * a.bands_per_img) * a.rows;
+            uint8_t* st = smem + s * stage_bytes;
+            BarArriveExpectTx(&full[s],
+                              a.x_box + (uint32_t)slices * a.dy_box);
+            TmaLoad4D(st, &tx, &full[s], c0, -1, r0 - 1, img);
+            for (int i = 0; i < slices; i++)
+                TmaLoad4D(st + a.x_bytes + i * a.dy_bytes, &tdy, &full[s],
+                          n0 + 32 * i, 0, r0, img);
+        }
+        for (int q = j > a.stages ? j - a.stages : 0; q < j; q++)
+            if (!BarWaitDrain(&full[q % a.stages], (q / a.stages) & 1))
+                Flag(cta_err, a.err);
+    } else if (warp == 1) {
+        // the whole warp walks the loop, one lane issues
+        const uint32_t idesc = InstrDescBf16(kTileM, a.bn, true, true);
+        // MN-major, 64-byte swizzle.  X: M rows 32 w + c are channel c at the
+        // position w further on (lbo one position); dY: slices lbo apart
+        const uint32_t base = SmemAddr(smem);
+        // a run of positions: an image row, or the band with its surplus
+        // columns where a row is no multiple of 16
+        const bool by_row = a.w % 16 == 0;
+        const int ksteps = ((by_row ? a.w : a.rows * a.pitch) + 15) / 16;
+        int j = 0;
+        for (int s = 0, phase = 0; j < nb; j++) {
+            const int r0 = (b0 + j) % a.bands_per_img * a.rows;
+            const int runs = by_row ? min(a.rows, a.h - r0) : 1;
+            if (!__all_sync(~0u, BarWait(&full[s], phase, cta_err))) {
+                if (lane == 0) Flag(cta_err, a.err);
+                break;
+            }
+            FenceAfterSync();
+            const uint32_t sx = base + s * stage_bytes;
+            const uint64_t db =
+                SmemDesc(sx + a.x_bytes, (uint32_t)a.dy_bytes, 8 * SW, SW);
+            if (ElectOne()) {
+                for (int dh = 0; dh < 3; dh++) {
+                    const uint64_t da = SmemDesc(sx + dh * a.pitch * SW, SW,
+                                                 8 * SW, SW);
+                    // a position on: four units of 16 bytes
+                    for (int r = 0; r < runs; r++)
+                        for (int k = 0; k < ksteps; k++) {
+                            const int at = 4 * (r * a.pitch + 16 * k);
+                            Mma(tmem + dh * a.bn, da + at, db + at, idesc,
+                                (j | r | k) != 0 ? 1u : 0u);
+                        }
+                }
+                Commit(&empty[s]);
+                if (j + 1 == nb) Commit(accum);
+            }
+            __syncwarp();
+            if (++s == a.stages) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+        if (j < nb && ElectOne()) Commit(accum);
+    }
+    __syncwarp();
+
+    const bool acc_ok = BarWaitDrain(accum, 0);
+    FenceAfterSync();
+    if (!acc_ok && threadIdx.x == 0) Flag(cta_err, a.err);
+    const bool store = acc_ok && *cta_err == 0;
+    // TMEM lane 32 w + c: tap column w (the fourth belongs to no tap)
+    const int ci = c0 + lane;
+    const bool row_ok = store && warp < 3 && ci < a.cin;
+    for (int dh = 0; dh < 3; dh++) {
+        const int tap = 3 * dh + warp;
+        for (int c = 0; c < a.bn; c += 16) {
+            float v[16];
+            TmemLoad16(tmem + ((uint32_t)(warp * 32) << 16) +
+                           (uint32_t)(dh * a.bn + c), v);
+            if (row_ok) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int co = n0 + c + i;
+                    if (co < a.cout)
+                        atomicAdd(a.dw + ((long long)co * 9 + tap) * a.cin + ci,
+                                  v[i]);
+                }
+            }
+            __syncwarp();
+        }
+    }
+
+    FenceBeforeSync();
+    __syncthreads();
+    if (warp == 2) {
+        FenceAfterSync();
+        TmemFree(tmem, a.tmem_cols);
+    }
+}
+
 }  // namespace nn
 }  // namespace mplb
 
@@ -976,6 +1138,74 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
     return true;
 }
 
+bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
+                     cudaStream_t stream, int* err_dev, std::string& err) {
+    WgradBandArgs a{};
+    a.w = x.w;
+    a.h = x.h;
+    a.pitch = x.w + 2;
+    a.cout = dy.c;
+    a.cin = x.c;
+    a.bn = 32 * std::min(4, (dy.c + 31) / 32);
+    const int slices = (x.c + 31) / 32, groups = (dy.c + a.bn - 1) / a.bn;
+    a.stages = 2;
+    // as many rows as leave room for two stages (a band reads two rows more
+    // than it has), and a band at least for every CTA: one CTA per SM (a
+    // training step 535 us in these kernels, with two per SM 701), and as many
+    // again for each further group of output channels, whose layers have few
+    // pixels: 256 -> 256 at 16^2 adds up 512 products per accumulator as tap by
+    // tap (2.9e-7 off the 64-bit sums); with 1024 it were 6.4e-7 (and 480 us)
+    const int per_slice = std::max(1, sm_count / slices);
+    a.rows = std::min(x.h, 250);
+    const auto fits = [&] {
+        a.x_bytes = WgradBandBytes((a.rows + 2) * a.pitch + 3);
+        a.dy_bytes = WgradBandBytes(a.rows * a.pitch);
+        return WgradBandSmemBytes(a) <= kSmemMax;
+    };
+    while (a.rows > 1 &&
+           (!fits() ||
+            (long long)x.nimg * ((x.h + a.rows - 1) / a.rows) < per_slice))
+        a.rows--;
+    if (!fits()) {
+        err = "weight gradient: a row does not fit in shared memory";
+        return false;
+    }
+    while (a.stages < 4) {
+        a.stages++;
+        if (WgradBandSmemBytes(a) > kSmemMax) {
+            a.stages--;
+            break;
+        }
+    }
+    a.x_box = (uint32_t)((a.rows + 2) * a.pitch * 64);
+    a.dy_box = (uint32_t)(a.rows * a.pitch * 64);
+    a.bands_per_img = (x.h + a.rows - 1) / a.rows;
+    a.bands_total = x.nimg * a.bands_per_img;
+    a.bands_per_cta = (a.bands_total + per_slice - 1) / per_slice;
+    a.tmem_cols = Pow2Cols(3 * a.bn);
+    a.dw = dw;
+    a.err = err_dev;
+    CUtensorMap tx, tdy;
+    if (!EncodeAct(&tx, x, 32, a.pitch, a.rows + 2, 64, err) ||
+        !EncodeAct(&tdy, dy, 32, a.pitch, a.rows, 64, err))
+        return false;
+    const dim3 grid((a.bands_total + a.bands_per_cta - 1) / a.bands_per_cta,
+                    slices, groups);
+    const int smem = ResidencySafeSmem(WgradBandSmemBytes(a), a.tmem_cols);
+    static cudaError_t attr = cudaFuncSetAttribute(
+        WgradBandKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    cudaError_t e = attr;
+    if (e == cudaSuccess) {
+        WgradBandKernel<<<grid, kConvThreads, smem, stream>>>(tx, tdy, a);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        err = std::string("weight-gradient launch: ") + cudaGetErrorString(e);
+        return false;
+    }
+    return true;
+}
+
 bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
                  int sm_count, cudaStream_t stream, int* err_dev,
                  std::string& err) {
@@ -986,6 +1216,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
         err = "weight-gradient shapes do not match";
         return false;
     }
+    if (taps == 9)
+        return LaunchWgradBand(dy, x, dw, sm_count, stream, err_dev, err);
     if (dy.c <= 64) {
         // few output channels: taps x input channels along M (WgradTKernel)
         CUtensorMap tx, tdy;

@@ -141,6 +141,35 @@ struct WgradTArgs {
     int* err;
 };
 
+// Weight gradient of a 3x3 convolution with its operands resident: a band of
+// image rows of one 32-channel slice of X (with its halo) and of bn channels of
+// dY in shared memory serve all nine taps.  Both are laid out W + 2 positions to
+// a row, dY's two surplus columns zero (TMA's fill), so the sum over pixels is a
+// sum over positions q and tap (dh, dw) pairs dY's position q with X's position
+// q + dh (W + 2) + dw.  M = 128 rows are the slice at four consecutive dw - three
+// of them taps: the operand descriptor steps one position between its 32-row
+// atoms - N = the output channels, one accumulator per dh.  CTAs sum ranges of
+// bands and add them with fp32 atomics.  The tap-by-tap kernels below moved X nine
+// times through L2 for it.
+struct WgradBandArgs {
+    int w, h;              // image
+    int pitch;             // positions per row: W + 2
+    int rows;              // of a band
+    int bands_per_img, bands_total, bands_per_cta;
+    int cout, cin;         // dW is [cout][9][cin]
+    int bn;                // UMMA N: 32 per slice of dY
+    int x_bytes, dy_bytes; // shared memory of a slice of a band
+    uint32_t x_box, dy_box;   // bytes of their TMA boxes
+    int stages;
+    int tmem_cols;         // >= 3 bn
+    float* dw;
+    int* err;
+};
+
+__global__ void WgradBandKernel(const __grid_constant__ CUtensorMap tx,
+                                const __grid_constant__ CUtensorMap tdy,
+                                WgradBandArgs a);
+
 template <int BK>
 __global__ void ConvBandKernel(const __grid_constant__ CUtensorMap ta,
                                const __grid_constant__ CUtensorMap tb,
@@ -176,6 +205,14 @@ inline int BandSmemBytes(int chunks, int chunk_bytes, int stages,
 }
 inline int WgradSmemBytes(int b_atoms, int stages) {
     return 1024 + stages * ((2 + b_atoms) * 16384) + 256;
+}
+// WgradBandKernel: a slice of so many positions, filled up to a multiple of 16
+// and the positions that the last ones' taps reach; the whole launch.
+inline int WgradBandBytes(int positions) {
+    return ((positions + 16) * 64 + 1023) / 1024 * 1024;
+}
+inline int WgradBandSmemBytes(const WgradBandArgs& a) {
+    return 1024 + a.stages * (a.x_bytes + a.bn / 32 * a.dy_bytes) + 256;
 }
 // WgradTKernel: per stage four 8 KiB X atoms and bn / 32 8 KiB dY atoms.
 inline int WgradTSmemBytes(int bn, int stages) {

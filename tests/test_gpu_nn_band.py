@@ -53,3 +53,39 @@ def test_band_forward(gpu_lib, shape, masked):
     scale = np.abs(ref).max()
     assert np.allclose(y[..., 8:8 + cout], ref, rtol=8e-3, atol=1e-3 * scale)
     assert not y[..., :8].any() and not y[..., 8 + cout:].any()
+
+
+# n, h, w, cout, cin: rows a band, output slices and groups, partial slices
+WGRAD_SHAPES = [
+    (1, 1, 128, 16, 16), (2, 3, 128, 32, 32), (1, 9, 128, 32, 96),
+    (3, 5, 128, 160, 32), (1, 2, 64, 64, 48), (3, 6, 64, 64, 192),
+    (1, 4, 32, 128, 64), (2, 36, 32, 128, 160), (9, 16, 16, 256, 128),
+    (40, 24, 16, 96, 256), (1, 16, 8, 96, 64), (2, 64, 2, 16, 32),
+    (1, 128, 1, 32, 16),
+]
+
+
+@pytest.mark.parametrize("shape", WGRAD_SHAPES)
+def test_band_wgrad(gpu_lib, shape):
+    """Sums of fp32 products of bf16 values over up to 15,360 pixels: rtol
+    1e-3 plus 1e-4 of the largest, as the shape tests' weight gradients; added
+    to what dw holds."""
+    from test_gpu_nn_conv import ref_wgrad
+    torch = _torch()
+    n, h, w, cout, cin = shape
+    rng = np.random.default_rng(h * 131 + w * 17 + cin)
+    # slices of wider buffers, whose other channels must not enter
+    x = bf16(rng.standard_normal((n, h, w, cin + 16))).cuda()
+    dy = bf16(rng.standard_normal((n, h, w, cout + 8))).cuda()
+    before = rng.standard_normal((cout, 9, cin)).astype(np.float32)
+    dw = torch.from_numpy(before).cuda()
+    torch.cuda.synchronize()
+    rc = gpu_lib.mplbnn_conv_wgrad(
+        ctypes.byref(view(dy, n, h, w, cout, cout + 8, 8)),
+        ctypes.byref(view(x, n, h, w, cin, cin + 16, 8)), 9, dw.data_ptr(),
+        None)
+    assert rc == 0, gpu_lib.mplbnn_error().decode()
+    ref = ref_wgrad(as64(dy)[..., 8:8 + cout], as64(x)[..., 8:8 + cin], 9)
+    got = dw.cpu().numpy().astype(np.float64) - before
+    scale = np.abs(ref).max()
+    assert np.allclose(got, ref, rtol=1e-3, atol=1e-4 * scale + 1e-6)
