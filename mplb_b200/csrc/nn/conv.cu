@@ -957,29 +957,41 @@ BandPlan PlanBand(int nimg, int H, int W, int cin, int cout, int bk,
     const int chunks = (cin + bk - 1) / bk, nkb = 9 * chunks;
     int bn = 128;
     while (cout % bn != 0) bn -= 16;
-    int tiles = std::max(1, std::min({4, (160 + bn / 2) / bn, per_img}));
+    int tiles = 1;
     const auto ctas = [&] {
         return (long long)nimg * ((per_img + tiles - 1) / tiles) * (cout / bn);
     };
-    while (tiles > 1 && ctas() < 2 * sm_count) tiles--;
     while (bn % 32 == 0 && bn > 32 && ctas() < sm_count) bn /= 2;
-    for (; tiles >= 1; tiles--) {
+    // Tiles of a CTA: its accumulators leave half of TMEM to another CTA.  An SM
+    // gets `per` CTAs, `per_sm` at a time, each such round costs about as much as
+    // a tile, and the fullest SM is the launch's time: 64 -> 64 at 64^2 (32
+    // images, 33 tiles each) 28 us with 1 tile, 25 with 2, 27 with 3; 32 -> 64
+    // 21, 19, 21 and with 4 17; 96 -> 32 at 128^2, 3 images, 19, 17, 12 and 15.
+    long long best = 0;
+    for (int most = std::min({4, bn <= 64 ? 4 : bn <= 96 ? 2 : 1, per_img});
+         tiles <= most; tiles++) {
         const int rows = (W == 128 ? (tiles - 1) * step + 127
                                    : pitch - 1 + (tiles - 1) * step + 127) /
                              pitch + 3;
-        if (rows > 256) continue;
+        if (rows > 256) break;
         const int chunk = BandChunkBytes(rows, pitch, bk);
         const int kb_bytes = bn * bk * 2;
         for (int per_sm = 2; per_sm >= 1; per_sm--) {
             const int room = std::min(kSmemPerSm / per_sm - 2048, kSmemMax);
             const int left = room - BandSmemBytes(chunks, chunk, 0, 0, bn, bk);
             if (left < std::min(3, nkb) * (kb_bytes + 16)) continue;
+            const long long per = (ctas() + sm_count - 1) / sm_count;
+            const long long cost = (per + per_sm - 1) / per_sm + per * tiles;
+            if (p.tiles > 0 && cost > best) break;
+            best = cost;
             // Waiting for a stage, committing it and forming its addresses
             // cost about 500 cycles, as much as 12 MMAs: a stage holds enough
-            // k-blocks for 32, or a third of what fits
+            // k-blocks for 72, or all that fit (the other CTA of the SM runs
+            // meanwhile): 96 -> 32 at 128^2 90 us, with 32 98; 128 -> 128 at
+            // 32^2 18.5, with a third of what fits 20.2
             const int mmas = tiles * (bk / 16);
-            p.group = std::min({nkb, (32 + mmas - 1) / mmas,
-                                std::max(1, left / 3 / (kb_bytes + 16))});
+            p.group = std::min({nkb, (72 + mmas - 1) / mmas,
+                                left / (kb_bytes + 16)});
             p.stages = std::min((nkb + p.group - 1) / p.group,
                                 left / (p.group * kb_bytes + 16));
             p.tiles = tiles;
@@ -987,7 +999,7 @@ BandPlan PlanBand(int nimg, int H, int W, int cin, int cout, int bk,
             p.rows = rows;
             p.smem = BandSmemBytes(chunks, chunk, p.stages,
                                    p.group * kb_bytes, bn, bk);
-            return p;
+            break;
         }
     }
     return p;
