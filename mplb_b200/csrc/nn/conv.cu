@@ -633,23 +633,23 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 
 // The weight gradient of a 3x3 convolution (see conv.cuh): one 32-channel slice
 // of the input, bn output channels, a range of bands of image rows.  Cold-cache
-// layer times (32 images), tap by tap in brackets: 96 -> 32 at 128^2 64 us (202),
-// 32 -> 32 30 (77), 192 -> 64 at 64^2 49 (116), 384 -> 128 at 32^2 51 (78), 128 ->
-// 128 28 (43).  Row by row a sum has as many terms as a tap's: over surplus columns, too,
+// layer times (32 images), tap by tap in brackets: 96 -> 32 at 128^2 61 us (202),
+// 32 -> 32 27 (77), 192 -> 64 at 64^2 43 (116), 384 -> 128 at 32^2 44 (78), 128 ->
+// 128 23 (43).  Row by row a sum has as many terms as a tap's: over surplus columns, too,
 // 256 -> 256 at 16^2 rounds 18/16 times as often, 3.0e-7 off the 64-bit sums in
 // place of 2.9e-7.  Rows under 16 pixels, which no layer of the network has, go over
 // them all the same: there a zero of dY meets a pixel of X that the tap does not use.
 __global__ void __launch_bounds__(kConvThreads, 1)
     WgradBandKernel(const __grid_constant__ CUtensorMap tx,
                     const __grid_constant__ CUtensorMap tdy,
+                    const __grid_constant__ CUtensorMap tdw,
                     WgradBandArgs a) {
     constexpr uint32_t SW = 64;   // bytes of a position: 32 channels
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = Align1024(smem_raw);
     const int slices = a.bn / 32;
     const uint32_t stage_bytes = a.x_bytes + slices * a.dy_bytes;
-    uint64_t* full =
-        reinterpret_cast<uint64_t*>(smem + a.stages * stage_bytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + WgradBandData(a));
     uint64_t* empty = full + a.stages;
     uint64_t* accum = empty + a.stages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
@@ -762,19 +762,31 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     const bool acc_ok = BarWaitDrain(accum, 0);
     FenceAfterSync();
     if (!acc_ok && threadIdx.x == 0) Flag(cta_err, a.err);
-    const bool store = acc_ok && *cta_err == 0;
-    // TMEM lane 32 w + c: tap column w (the fourth belongs to no tap)
+    const bool store = __all_sync(~0u, acc_ok && *cta_err == 0);
+    // TMEM lane 32 w + c: tap column w (the fourth belongs to no tap).  The
+    // stages are read by now: each warp lays its tap's 32 x bn sums out there and
+    // one bulk reduction adds them to dW, clipped at its edges.  Lane by lane, at
+    // about one atomic a cycle and SM, this took most of the layers of few pixels
+    // and many channels: 256 -> 256 at 16^2 56 us
+    // -> 34, a training step 535 us in this kernel -> 413.
     const int ci = c0 + lane;
-    const bool row_ok = store && warp < 3 && ci < a.cin;
-    for (int dh = 0; dh < 3; dh++) {
+    const uint32_t row = tmem + ((uint32_t)(warp * 32) << 16);
+    float* out = reinterpret_cast<float*>(smem) + warp * a.bn * 32;
+    for (int dh = 0; dh < 3 && warp < 3; dh++) {
         const int tap = 3 * dh + warp;
-        for (int c = 0; c < a.bn; c += 16) {
-            float v[16];
-            TmemLoad16(tmem + ((uint32_t)(warp * 32) << 16) +
-                           (uint32_t)(dh * a.bn + c), v);
-            if (row_ok) {
+        if (a.bulk && dh > 0) {
+            if (lane == 0) BulkWaitRead();
+            __syncwarp();
+        }
+        for (int c = 0; c < a.bn; c += 32) {
+            float v[32];
+            TmemLoad32(row + (uint32_t)(dh * a.bn + c), v);
+            if (a.bulk && store) {
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
+                for (int i = 0; i < 32; i++) out[(c + i) * 32 + lane] = v[i];
+            } else if (store && ci < a.cin) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) {
                     const int co = n0 + c + i;
                     if (co < a.cout)
                         atomicAdd(a.dw + ((long long)co * 9 + tap) * a.cin + ci,
@@ -783,7 +795,16 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             }
             __syncwarp();
         }
+        if (a.bulk && store) {
+            FenceProxyAsync();
+            __syncwarp();
+            if (lane == 0) {
+                TmaAdd3D(&tdw, out, c0, tap, n0);
+                BulkCommit();
+            }
+        }
     }
+    if (lane == 0) BulkWaitRead();
 
     FenceBeforeSync();
     __syncthreads();
@@ -850,6 +871,31 @@ bool EncodeAct(CUtensorMap* m, const View& v, int box_c, int box_w, int box_h,
         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         err = "tensor map of an activation view rejected (CUresult " +
+              std::to_string((int)r) + ")";
+        return false;
+    }
+    return true;
+}
+
+// fp32 dW [cout][9][cin]: boxes of 32 input channels of one tap x bn output
+// channels.
+bool EncodeWeightGrad(CUtensorMap* m, float* dw, int cin, int cout, int bn,
+                      std::string& err) {
+    EncodeTiledFn enc = Encoder();
+    if (enc == nullptr) {
+        err = "cuTensorMapEncodeTiled is not available";
+        return false;
+    }
+    const cuuint64_t dims[3] = {(cuuint64_t)cin, 9, (cuuint64_t)cout};
+    const cuuint64_t strides[2] = {(cuuint64_t)cin * 4, (cuuint64_t)cin * 36};
+    const cuuint32_t box[3] = {32, 1, (cuuint32_t)bn};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc(
+        m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dw, dims, strides, box, estr,
+        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        err = "tensor map of a weight gradient rejected (CUresult " +
               std::to_string((int)r) + ")";
         return false;
     }
@@ -941,11 +987,10 @@ struct BandPlan {
     int smem = 0;
 };
 
-// Tiles and output channels of a CTA: two CTAs per SM of about 160
-// accumulator columns measured best over the network's layers (32 images,
-// cold L2, against tap by tap: 32 -> 32 channels at 128^2 31 us, was 48; 64 ->
-// 64 at 64^2 24, was 33; 128 -> 128 at 32^2 19, was 26), with fewer tiles and
-// then fewer channels while the GPU is not full.  Above 128 input channels the
+// Tiles and output channels of a CTA (cold-L2 times of the network's layers, 32
+// images, against tap by tap: 32 -> 32 channels at 128^2 33 us, was 48; 64 -> 64
+// at 64^2 25, was 33; 128 -> 128 at 32^2 20, was 26), with fewer output channels
+// while the GPU is not full.  Above 128 input channels the
 // band fills the shared memory that the weights stream through (192 -> 64 at
 // 64^2 64 us, was 61; 384 -> 128 at 32^2 108, was 53).
 BandPlan PlanBand(int nimg, int H, int W, int cin, int cout, int bk,
@@ -1163,11 +1208,14 @@ bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
     a.stages = 2;
     // as many rows as leave room for two stages (a band reads two rows more
     // than it has), and a band at least for every CTA: one CTA per SM (a
-    // training step 535 us in these kernels, with two per SM 701), and as many
-    // again for each further group of output channels, whose layers have few
-    // pixels: 256 -> 256 at 16^2 adds up 512 products per accumulator as tap by
-    // tap (2.9e-7 off the 64-bit sums); with 1024 it were 6.4e-7 (and 480 us)
-    const int per_slice = std::max(1, sm_count / slices);
+    // training step, with an atomic per lane, 535 us in these kernels, with two
+    // per SM 701), and as many again for each further group of output channels,
+    // whose layers have few pixels: 256 -> 256 at 16^2 adds up 512 products per
+    // accumulator as tap by tap (2.9e-7 off the 64-bit sums); with 1024 it were
+    // 6.4e-7.  A CTA has at least 128 pixels to pay for its sums' way out.
+    const int per_slice = std::max(
+        1, (int)std::min<long long>(sm_count / slices,
+                                    (long long)x.nimg * x.h * x.w / 128));
     a.rows = std::min(x.h, 250);
     const auto fits = [&] {
         a.x_bytes = WgradBandBytes((a.rows + 2) * a.pitch + 3);
@@ -1197,9 +1245,13 @@ bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
     a.tmem_cols = Pow2Cols(3 * a.bn);
     a.dw = dw;
     a.err = err_dev;
-    CUtensorMap tx, tdy;
+    CUtensorMap tx, tdy, tdw{};
     if (!EncodeAct(&tx, x, 32, a.pitch, a.rows + 2, 64, err) ||
         !EncodeAct(&tdy, dy, 32, a.pitch, a.rows, 64, err))
+        return false;
+    // bulk reductions take 16-byte aligned rows; elsewhere one atomic per lane
+    a.bulk = reinterpret_cast<uintptr_t>(dw) % 16 == 0 && x.c % 4 == 0 ? 1 : 0;
+    if (a.bulk && !EncodeWeightGrad(&tdw, dw, x.c, dy.c, a.bn, err))
         return false;
     const dim3 grid((a.bands_total + a.bands_per_cta - 1) / a.bands_per_cta,
                     slices, groups);
@@ -1208,7 +1260,7 @@ bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
         WgradBandKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     cudaError_t e = attr;
     if (e == cudaSuccess) {
-        WgradBandKernel<<<grid, kConvThreads, smem, stream>>>(tx, tdy, a);
+        WgradBandKernel<<<grid, kConvThreads, smem, stream>>>(tx, tdy, tdw, a);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

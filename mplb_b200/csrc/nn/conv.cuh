@@ -149,7 +149,7 @@ struct WgradTArgs {
 // q + dh (W + 2) + dw.  M = 128 rows are the slice at four consecutive dw - three
 // of them taps: the operand descriptor steps one position between its 32-row
 // atoms - N = the output channels, one accumulator per dh.  CTAs sum ranges of
-// bands and add them with fp32 atomics.  The tap-by-tap kernels below moved X nine
+// bands and add them to dW in fp32 (bulk reductions).  The tap-by-tap kernels below moved X nine
 // times through L2 for it.
 struct WgradBandArgs {
     int w, h;              // image
@@ -162,12 +162,14 @@ struct WgradBandArgs {
     uint32_t x_box, dy_box;   // bytes of their TMA boxes
     int stages;
     int tmem_cols;         // >= 3 bn
+    int bulk;              // dW takes bulk reductions
     float* dw;
     int* err;
 };
 
 __global__ void WgradBandKernel(const __grid_constant__ CUtensorMap tx,
                                 const __grid_constant__ CUtensorMap tdy,
+                                const __grid_constant__ CUtensorMap tdw,
                                 WgradBandArgs a);
 
 template <int BK>
@@ -211,8 +213,14 @@ inline int WgradSmemBytes(int b_atoms, int stages) {
 inline int WgradBandBytes(int positions) {
     return ((positions + 16) * 64 + 1023) / 1024 * 1024;
 }
+// The stages, in whose place the sums of three taps are laid out at the end.
+__host__ __device__ inline int WgradBandData(const WgradBandArgs& a) {
+    const int stages = a.stages * (a.x_bytes + a.bn / 32 * a.dy_bytes);
+    const int sums = 3 * a.bn * 32 * 4;
+    return stages > sums ? stages : sums;
+}
 inline int WgradBandSmemBytes(const WgradBandArgs& a) {
-    return 1024 + a.stages * (a.x_bytes + a.bn / 32 * a.dy_bytes) + 256;
+    return 1024 + WgradBandData(a) + 256;
 }
 // WgradTKernel: per stage four 8 KiB X atoms and bn / 32 8 KiB dY atoms.
 inline int WgradTSmemBytes(int bn, int stages) {

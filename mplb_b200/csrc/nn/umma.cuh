@@ -40,6 +40,26 @@ using tma::SmemAddr;
 using tma::TmaLoad2D;
 using tma::TmaLoad4D;
 
+// ---- bulk reductions --------------------------------------------------------
+
+// Adds the fp32 box at `src` (shared memory, written behind FenceProxyAsync) to
+// the tensor's memory from (x, y, z) on; elements beyond its extents are left.
+__device__ __forceinline__ void TmaAdd3D(const CUtensorMap* m, const void* src,
+                                         int x, int y, int z) {
+    asm volatile(
+        "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group "
+        "[%0, {%1, %2, %3}], [%4];" ::"l"(m),
+        "r"(x), "r"(y), "r"(z), "r"(SmemAddr(src))
+        : "memory");
+}
+__device__ __forceinline__ void BulkCommit() {
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// The thread's reductions have read their shared memory.
+__device__ __forceinline__ void BulkWaitRead() {
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
 // ---- tensor memory ---------------------------------------------------------
 
 // Whole warp: allocates `ncols` TMEM columns (power of two >= 32) and writes

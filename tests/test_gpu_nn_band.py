@@ -65,8 +65,9 @@ WGRAD_SHAPES = [
 ]
 
 
+@pytest.mark.parametrize("shift", [0, 1])
 @pytest.mark.parametrize("shape", WGRAD_SHAPES)
-def test_band_wgrad(gpu_lib, shape):
+def test_band_wgrad(gpu_lib, shape, shift):
     """Sums of fp32 products of bf16 values over up to 15,360 pixels: rtol
     1e-3 plus 1e-4 of the largest, as the shape tests' weight gradients; added
     to what dw holds."""
@@ -78,7 +79,11 @@ def test_band_wgrad(gpu_lib, shape):
     x = bf16(rng.standard_normal((n, h, w, cin + 16))).cuda()
     dy = bf16(rng.standard_normal((n, h, w, cout + 8))).cuda()
     before = rng.standard_normal((cout, 9, cin)).astype(np.float32)
-    dw = torch.from_numpy(before).cuda()
+    # added by bulk reductions, one atomic per lane off 16-byte alignment; what
+    # lies around it stays
+    mem = torch.full((before.size + 8,), 7.0, device="cuda")
+    dw = mem[4 + shift:4 + shift + before.size].view(before.shape)
+    dw.copy_(torch.from_numpy(before))
     torch.cuda.synchronize()
     rc = gpu_lib.mplbnn_conv_wgrad(
         ctypes.byref(view(dy, n, h, w, cout, cout + 8, 8)),
@@ -89,3 +94,4 @@ def test_band_wgrad(gpu_lib, shape):
     got = dw.cpu().numpy().astype(np.float64) - before
     scale = np.abs(ref).max()
     assert np.allclose(got, ref, rtol=1e-3, atol=1e-4 * scale + 1e-6)
+    assert (mem[:4 + shift] == 7).all() and (mem[4 + shift + before.size:] == 7).all()
