@@ -1,5 +1,6 @@
 // Tensor-core convolution kernels (see conv.cuh for the formulation).
 #include "conv.cuh"
+#include "launch_next.cuh"
 #include "umma.cuh"
 
 namespace mplb {
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         PrefetchTmap(&tb);
     }
     if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    GridWait();
     FenceBeforeSync();
     __syncthreads();
     FenceAfterSync();
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         PrefetchTmap(&tb);
     }
     if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    GridWait();
     for (int n = threadIdx.x; n < a.bn; n += kConvThreads)
         bias[n] = a.bias != nullptr ? a.bias[n0 + n] : 0.0f;
     FenceBeforeSync();
@@ -424,6 +427,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         PrefetchTmap(&tb);
     }
     if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    GridWait();
     FenceBeforeSync();
     __syncthreads();
     FenceAfterSync();
@@ -538,6 +542,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         PrefetchTmap(&tdy);
     }
     if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
+    GridWait();
     FenceBeforeSync();
     __syncthreads();
     FenceAfterSync();
@@ -685,6 +690,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 reinterpret_cast<uint4*>(at)[e] = make_uint4(0, 0, 0, 0);
         }
     FenceProxyAsync();
+    GridWait();
     FenceBeforeSync();
     __syncthreads();
     FenceAfterSync();
@@ -1088,9 +1094,11 @@ bool LaunchConvBand(const View& x, const void* w, const BandPlan& p, int bk,
     cudaError_t e = bk == 64 ? SetBandSmemAttr<64>() : SetBandSmemAttr<32>();
     if (e == cudaSuccess) {
         if (bk == 64)
-            ConvBandKernel<64><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+            LaunchNext(ConvBandKernel<64>, grid, kConvThreads, smem, stream,
+                       ta, tb, a);
         else
-            ConvBandKernel<32><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+            LaunchNext(ConvBandKernel<32>, grid, kConvThreads, smem, stream,
+                       ta, tb, a);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -1181,11 +1189,13 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
     if (bk == 64) {
         e = SetSmemAttr<64>();
         if (e == cudaSuccess)
-            ConvKernel<64><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+            LaunchNext(ConvKernel<64>, grid, kConvThreads, smem, stream,
+                       ta, tb, a);
     } else {
         e = SetSmemAttr<32>();
         if (e == cudaSuccess)
-            ConvKernel<32><<<grid, kConvThreads, smem, stream>>>(ta, tb, a);
+            LaunchNext(ConvKernel<32>, grid, kConvThreads, smem, stream,
+                       ta, tb, a);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1260,7 +1270,8 @@ bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
         WgradBandKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     cudaError_t e = attr;
     if (e == cudaSuccess) {
-        WgradBandKernel<<<grid, kConvThreads, smem, stream>>>(tx, tdy, tdw, a);
+        LaunchNext(WgradBandKernel, grid, kConvThreads, smem, stream, tx, tdy,
+                   tdw, a);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {
@@ -1314,8 +1325,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
                                            t.tmem_cols);
         cudaError_t e = SetWgradTSmemAttr();
         if (e == cudaSuccess)
-            WgradTKernel<<<dim3(mtiles, splits), kConvThreads, smem, stream>>>(
-                tx, tdy, t);
+            LaunchNext(WgradTKernel, dim3(mtiles, splits), kConvThreads, smem,
+                       stream, tx, tdy, t);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) {
             err = std::string("weight-gradient launch: ") +
@@ -1353,8 +1364,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
                                        a.tmem_cols);
     cudaError_t e = SetWgradSmemAttr();
     if (e == cudaSuccess)
-        WgradKernel<<<dim3(blocks, splits), kConvThreads, smem, stream>>>(
-            ta, tb, a);
+        LaunchNext(WgradKernel, dim3(blocks, splits), kConvThreads, smem, stream,
+                   ta, tb, a);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
         err = std::string("weight-gradient launch: ") + cudaGetErrorString(e);

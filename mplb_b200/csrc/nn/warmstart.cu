@@ -26,6 +26,7 @@
 
 #include "../../../include/mplbnn.h"
 #include "conv_host.h"
+#include "launch_next.cuh"
 
 namespace mplb {
 namespace nn {
@@ -96,6 +97,7 @@ __device__ __forceinline__ void St8(bf16* base, long long pix, long long ps,
 // Input planes of one pixel: cond0..2, x, y (node centres), zeros.
 __global__ void InputKernel(const float* __restrict__ cond, int n,
                             bf16* __restrict__ xin) {
+    GridWait();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (long long)n * kGrid * kGrid) return;
     const int img = (int)(p / (kGrid * kGrid));
@@ -160,6 +162,7 @@ __device__ __forceinline__ void SumChildren(const bf16* __restrict__ src,
 __global__ void PoolKernel(const bf16* __restrict__ src, long long sps,
                            bf16* __restrict__ dst, long long dps, unsigned n,
                            int lw, int lg) {
+    GridWait();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const EwIndex i = EwAt(t, lw, lg);
@@ -174,6 +177,7 @@ __global__ void PoolKernel(const bf16* __restrict__ src, long long sps,
 __global__ void UpsampleKernel(const bf16* __restrict__ src, long long sps,
                                bf16* __restrict__ dst, long long dps,
                                unsigned n, int lw, int lg) {
+    GridWait();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const EwIndex i = EwAt(t, lw, lg);
@@ -199,6 +203,7 @@ __global__ void UpBwdKernel(const bf16* __restrict__ gsrc, long long gps,
                             const bf16* __restrict__ act, long long aps,
                             bf16* __restrict__ gdst, long long dps, unsigned n,
                             int lw, int lg) {
+    GridWait();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const EwIndex i = EwAt(t, lw, lg);
@@ -215,6 +220,7 @@ __global__ void SkipBwdKernel(const bf16* __restrict__ gskip, long long sps,
                               const bf16* __restrict__ act, long long aps,
                               bf16* __restrict__ gdst, long long dps,
                               unsigned n, int lw, int lg) {
+    GridWait();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const EwIndex i = EwAt(t, lw, lg);
@@ -236,6 +242,7 @@ __global__ void __launch_bounds__(kEw)
     LossKernel(const float* __restrict__ pred,
                const float* __restrict__ target, long long npix, float scale,
                bf16* __restrict__ dpred, double* __restrict__ loss) {
+    GridWait();
     __shared__ double part[kEw / 32];
     double s = 0.0;
     for (long long p = (long long)blockIdx.x * kEw + threadIdx.x; p < npix;
@@ -269,6 +276,7 @@ __global__ void __launch_bounds__(kEw)
 __global__ void __launch_bounds__(kEw)
     BiasGradKernel(const bf16* __restrict__ dz, long long ps, long long npix,
                    int c, float* __restrict__ db) {
+    GridWait();
     __shared__ float part[kEw * 8];
     const int groups = c / 8;               // 2..32, divides kEw
     const int lanes = kEw / groups;
@@ -319,6 +327,7 @@ __global__ void AdamKernel(float* __restrict__ w, const float* __restrict__ g,
                            bf16* __restrict__ wf, bf16* __restrict__ wd,
                            const __grid_constant__ ParamLayout l, int n,
                            float lr_t, float b1, float b2, float eps) {
+    GridWait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -350,6 +359,7 @@ __global__ void __launch_bounds__(kEw)
                  const float* __restrict__ cond,
                  const float* __restrict__ target, float* __restrict__ cond_to,
                  float* __restrict__ target_to) {
+    GridWait();
     constexpr int kPer = kGrid * kGrid * 3;
     const long long from = index.at[blockIdx.y], to = blockIdx.y;
     if (blockIdx.x == 0 && threadIdx.x < 3)
@@ -363,6 +373,7 @@ __global__ void __launch_bounds__(kEw)
 
 __global__ void CompactKernel(const float* __restrict__ pred, long long npix,
                               float* __restrict__ out) {
+    GridWait();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
     for (int c = 0; c < 3; c++) out[p * 3 + c] = pred[p * kOutCh + c];
@@ -591,9 +602,9 @@ int Wgrad(mplbnn_net* net, int l, const View& dz, const View& x) {
     const int c = dz.c;
     const int blocks =
         (int)std::min<long long>((npix + 63) / 64, 2 * net->sm_count);
-    BiasGradKernel<<<blocks, kEw, 0, net->stream>>>(
-        static_cast<const bf16*>(dz.ptr), dz.ps, npix, c,
-        net->grads + net->b_off[l]);
+    LaunchNext(BiasGradKernel, blocks, kEw, 0, net->stream,
+               static_cast<const bf16*>(dz.ptr), dz.ps, npix, c,
+               net->grads + net->b_off[l]);
     NCK(cudaGetLastError());
     return kOK;
 }
@@ -640,33 +651,33 @@ int Log2(int v) {
 void Pool(mplbnn_net* net, const bf16* src, int sps, bf16* dst, int n, int s,
           int c) {
     const unsigned t = EwThreads(n, s, c);
-    PoolKernel<<<Blocks(t), kEw, 0, net->stream>>>(src, sps, dst, c, t,
-                                                   Log2(s), Log2(c / 8));
+    LaunchNext(PoolKernel, Blocks(t), kEw, 0, net->stream, src, sps, dst, c, t,
+               Log2(s), Log2(c / 8));
 }
 void Upsample(mplbnn_net* net, const bf16* src, bf16* dst, int dps, int n,
               int s, int c) {
     const unsigned t = EwThreads(n, s, c);
-    UpsampleKernel<<<Blocks(t), kEw, 0, net->stream>>>(src, c, dst, dps, t,
-                                                       Log2(s), Log2(c / 8));
+    LaunchNext(UpsampleKernel, Blocks(t), kEw, 0, net->stream, src, c, dst, dps,
+               t, Log2(s), Log2(c / 8));
 }
 void UpBwd(mplbnn_net* net, const bf16* gsrc, int gps, const bf16* act,
            bf16* gdst, int n, int s, int c) {
     const unsigned t = EwThreads(n, s, c);
-    UpBwdKernel<<<Blocks(t), kEw, 0, net->stream>>>(
-        gsrc, gps, act, c, gdst, c, t, Log2(s), Log2(c / 8));
+    LaunchNext(UpBwdKernel, Blocks(t), kEw, 0, net->stream, gsrc, gps, act, c,
+               gdst, c, t, Log2(s), Log2(c / 8));
 }
 void SkipBwd(mplbnn_net* net, const bf16* gskip, int ps, const bf16* gpool,
              const bf16* act, bf16* gdst, int n, int s, int c) {
     const unsigned t = EwThreads(n, s, c);
-    SkipBwdKernel<<<Blocks(t), kEw, 0, net->stream>>>(
-        gskip, ps, gpool, c, act, ps, gdst, c, t, Log2(s), Log2(c / 8));
+    LaunchNext(SkipBwdKernel, Blocks(t), kEw, 0, net->stream, gskip, ps, gpool,
+               c, act, ps, gdst, c, t, Log2(s), Log2(c / 8));
 }
 
 int Forward(mplbnn_net* net, const float* cond, int n) {
     const int S0 = 128, S1 = 64, S2 = 32, S3 = 16;
     cudaStream_t st = net->stream;
-    InputKernel<<<Blocks((long long)n * S0 * S0), kEw, 0, st>>>(cond, n,
-                                                                 net->xin);
+    LaunchNext(InputKernel, Blocks((long long)n * S0 * S0), kEw, 0, st,
+               cond, n, net->xin);
     NCK(cudaGetLastError());
     // encoder
     RET(Conv(net, 0, V(net->xin, n, S0, 32), V(net->e0a, n, S0, 32), false));
@@ -706,10 +717,9 @@ int Backward(mplbnn_net* net, const float* target, int n) {
     const long long npix = (long long)n * S0 * S0;
     NCK(cudaMemsetAsync(net->grads, 0, net->np * sizeof(float), st));
     NCK(cudaMemsetAsync(net->loss_dev, 0, sizeof(double), st));
-    LossKernel<<<std::min<unsigned>(Blocks(npix), 4 * net->sm_count), kEw, 0,
-                 st>>>(
-        net->pred, target, npix, (float)(2.0 / (3.0 * (double)npix)),
-        net->dpred, net->loss_dev);
+    LaunchNext(LossKernel, std::min<unsigned>(Blocks(npix), 4 * net->sm_count),
+               kEw, 0, st, net->pred, target, npix,
+               (float)(2.0 / (3.0 * (double)npix)), net->dpred, net->loss_dev);
     NCK(cudaGetLastError());
     // decoder, level 0
     const View dpred = V(net->dpred, n, S0, kOutCh);
@@ -1065,7 +1075,8 @@ int mplbnn_forward(mplbnn_net* net, const float* cond, int n, float* pred) {
     if (!cond || !pred) return Fail(net, kInvalid, "null pointer");
     RET(Forward(net, cond, n));
     const long long npix = (long long)n * kGrid * kGrid;
-    CompactKernel<<<Blocks(npix), kEw, 0, net->stream>>>(net->pred, npix, pred);
+    LaunchNext(CompactKernel, Blocks(npix), kEw, 0, net->stream,
+               net->pred, npix, pred);
     NCK(cudaGetLastError());
     return Sync(net);
 }
@@ -1082,9 +1093,9 @@ int mplbnn_loss_grad(mplbnn_net* net, const float* cond, const float* target,
             const int m = std::min(n - i0, (int)SampleIndex::kMost);
             SampleIndex at{};
             std::copy(index + i0, index + i0 + m, at.at);
-            GatherKernel<<<dim3(16, m), kEw, 0, net->stream>>>(
-                at, cond, target, net->cond_buf + 3 * i0,
-                net->target_buf + per * i0);
+            LaunchNext(GatherKernel, dim3(16, m), kEw, 0, net->stream, at, cond,
+                       target, net->cond_buf + 3 * i0,
+                       net->target_buf + per * i0);
             NCK(cudaGetLastError());
         }
         cond = net->cond_buf;
@@ -1109,9 +1120,9 @@ int mplbnn_adam_step(mplbnn_net* net, float lr, float beta1, float beta2,
     const double bc1 = 1.0 - std::pow((double)beta1, (double)net->step);
     const double bc2 = 1.0 - std::pow((double)beta2, (double)net->step);
     const float lr_t = (float)(lr * std::sqrt(bc2) / bc1);
-    AdamKernel<<<Blocks(net->np), kEw, 0, net->stream>>>(
-        net->params, net->grads, net->m, net->v, net->wf, net->wd, Layout(net),
-        (int)net->np, lr_t, beta1, beta2, eps);
+    LaunchNext(AdamKernel, Blocks(net->np), kEw, 0, net->stream, net->params,
+               net->grads, net->m, net->v, net->wf, net->wd, Layout(net),
+               (int)net->np, lr_t, beta1, beta2, eps);
     NCK(cudaGetLastError());
     return kOK;
 }
