@@ -32,7 +32,8 @@
 // the band.  Tap and slice follow each other as in ConvKernel, so the sums are
 // the same bits.
 //
-// WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
+// The weight gradient of a 3x3 convolution is WgradBandKernel's (below); the two
+// that follow serve 1x1 convolutions.  WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
 // X[p + offset(t)][c]: M = 128 output channels, N = input channels, K = a
 // range of 128-pixel blocks (split over CTAs, accumulated with fp32 atomics).
 // Both operands arrive pixel-major with channels contiguous, i.e. MN-major,
@@ -149,8 +150,8 @@ struct WgradTArgs {
 // q + dh (W + 2) + dw.  M = 128 rows are the slice at four consecutive dw - three
 // of them taps: the operand descriptor steps one position between its 32-row
 // atoms - N = the output channels, one accumulator per dh.  CTAs sum ranges of
-// bands and add them to dW in fp32 (bulk reductions).  The tap-by-tap kernels below moved X nine
-// times through L2 for it.
+// bands and add them to dW in fp32 (bulk reductions).  Tap by tap X moved nine times through L2
+// for it.
 struct WgradBandArgs {
     int w, h;              // image
     int pitch;             // positions per row: W + 2
