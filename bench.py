@@ -373,9 +373,12 @@ def run_cavities(args, rank, world, local):
                                   "(LPT on nodes)"},
         "timing": {"repetitions": len(times),
                    "statistic": "median over repetitions of K timed steps"},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "issue", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "bytes_per_node": 72,
+                     "note": "72 B per node update as if every step went "
+                             "through HBM; steps of one call run in shared "
+                             "memory",
                      "traffic": None},
         "tuning": tuned["tuning"],
         "autotune": [{"mlups": round(r["mlups"], 1),
