@@ -29,7 +29,7 @@ HEADERS = [os.path.join(CSRC, h) for h in ("kernels.cuh", "lattice.h",
                                             "batch_kernels.cuh",
                                             "batch_resident.cuh", "tma.cuh",
                                             "nn/umma.cuh", "nn/conv.cuh",
-                                            "nn/conv_host.h",
+                                            "nn/conv_host.h", "nn/conv_plan.h",
                                             "nn/launch_next.cuh")] + [
     os.path.join(HERE, "..", "include", h) for h in ("mplbgpu.h", "mplbnn.h")]
 ARCH = "-gencode=arch=compute_100a,code=sm_100a"

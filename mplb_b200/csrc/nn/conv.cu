@@ -640,10 +640,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // of the input, bn output channels, a range of bands of image rows.  Cold-cache
 // layer times (32 images), tap by tap in brackets: 96 -> 32 at 128^2 61 us (202),
 // 32 -> 32 27 (77), 192 -> 64 at 64^2 43 (116), 384 -> 128 at 32^2 44 (78), 128 ->
-// 128 23 (43).  Row by row a sum has as many terms as a tap's: over surplus columns, too,
-// 256 -> 256 at 16^2 rounds 18/16 times as often, 3.0e-7 off the 64-bit sums in
-// place of 2.9e-7.  Rows under 16 pixels, which no layer of the network has, go over
-// them all the same: there a zero of dY meets a pixel of X that the tap does not use.
+// 128 23 (43).  Row by row a sum has the terms of a tap's and no others: over
+// surplus columns, too, 256 -> 256 at 16^2 rounds 18/16 times as often, 3.0e-7 off
+// the 64-bit sums in place of 2.9e-7, and a pixel that a tap does not use enters it
+// times zero.  So rows are 16 pixels or a multiple (kWgradBandWidth).
 __global__ void __launch_bounds__(kConvThreads, 1)
     WgradBandKernel(const __grid_constant__ CUtensorMap tx,
                     const __grid_constant__ CUtensorMap tdy,
@@ -678,18 +678,6 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         PrefetchTmap(&tdy);
     }
     if (warp == 2) TmemAlloc(tmem_slot, a.tmem_cols);
-    // the positions past a band's last row, which no copy writes, are zero:
-    // they fill up the last 16 positions of the sum
-    for (int s = 0; s < a.stages; s++)
-        for (int i = 0; i <= slices; i++) {
-            uint8_t* at = smem + s * stage_bytes +
-                          (i == 0 ? 0 : a.x_bytes + (i - 1) * a.dy_bytes);
-            const int from = (int)(i == 0 ? a.x_box : a.dy_box) / 16;
-            const int to = (i == 0 ? a.x_bytes : a.dy_bytes) / 16;
-            for (int e = from + (int)threadIdx.x; e < to; e += kConvThreads)
-                reinterpret_cast<uint4*>(at)[e] = make_uint4(0, 0, 0, 0);
-        }
-    FenceProxyAsync();
     GridWait();
     FenceBeforeSync();
     __syncthreads();
@@ -724,14 +712,11 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         // MN-major, 64-byte swizzle.  X: M rows 32 w + c are channel c at the
         // position w further on (lbo one position); dY: slices lbo apart
         const uint32_t base = SmemAddr(smem);
-        // a run of positions: an image row, or the band with its surplus
-        // columns where a row is no multiple of 16
-        const bool by_row = a.w % 16 == 0;
-        const int ksteps = ((by_row ? a.w : a.rows * a.pitch) + 15) / 16;
+        const int ksteps = a.w / 16;   // of an image row
         int j = 0;
         for (int s = 0, phase = 0; j < nb; j++) {
             const int r0 = (b0 + j) % a.bands_per_img * a.rows;
-            const int runs = by_row ? min(a.rows, a.h - r0) : 1;
+            const int runs = min(a.rows, a.h - r0);
             if (!__all_sync(~0u, BarWait(&full[s], phase, cta_err))) {
                 if (lane == 0) Flag(cta_err, a.err);
                 break;
@@ -831,6 +816,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 #include <string>
 
 #include "conv_host.h"
+#include "conv_plan.h"
 
 namespace mplb {
 namespace nn {
@@ -1291,7 +1277,7 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
         err = "weight-gradient shapes do not match";
         return false;
     }
-    if (taps == 9)
+    if (taps == 9 && x.w >= kWgradBandWidth)
         return LaunchWgradBand(dy, x, dw, sm_count, stream, err_dev, err);
     if (dy.c <= 64) {
         // few output channels: taps x input channels along M (WgradTKernel)

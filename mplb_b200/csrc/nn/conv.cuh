@@ -32,8 +32,9 @@
 // the band.  Tap and slice follow each other as in ConvKernel, so the sums are
 // the same bits.
 //
-// The weight gradient of a 3x3 convolution is WgradBandKernel's (below); the two
-// that follow serve 1x1 convolutions.  WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
+// The weight gradient of a 3x3 convolution over rows of 16 pixels or more is
+// WgradBandKernel's (below); the two that follow serve narrower rows and 1x1
+// convolutions.  WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
 // X[p + offset(t)][c]: M = 128 output channels, N = input channels, K = a
 // range of 128-pixel blocks (split over CTAs, accumulated with fp32 atomics).
 // Both operands arrive pixel-major with channels contiguous, i.e. MN-major,
@@ -145,9 +146,8 @@ struct WgradTArgs {
 // Weight gradient of a 3x3 convolution with its operands resident: a band of
 // image rows of one 32-channel slice of X (with its halo) and of bn channels of
 // dY in shared memory serve all nine taps.  Both are laid out W + 2 positions to
-// a row, dY's two surplus columns zero (TMA's fill), so the sum over pixels is a
-// sum over positions q and tap (dh, dw) pairs dY's position q with X's position
-// q + dh (W + 2) + dw.  M = 128 rows are the slice at four consecutive dw - three
+// a row, and tap (dh, dw) pairs dY's position q with X's position
+// q + dh (W + 2) + dw, for the W positions of each row.  M = 128 rows are the slice at four consecutive dw - three
 // of them taps: the operand descriptor steps one position between its 32-row
 // atoms - N = the output channels, one accumulator per dh.  CTAs sum ranges of
 // bands and add them to dW in fp32 (bulk reductions).  Tap by tap X moved nine times through L2
@@ -209,10 +209,9 @@ inline int BandSmemBytes(int chunks, int chunk_bytes, int stages,
 inline int WgradSmemBytes(int b_atoms, int stages) {
     return 1024 + stages * ((2 + b_atoms) * 16384) + 256;
 }
-// WgradBandKernel: a slice of so many positions, filled up to a multiple of 16
-// and the positions that the last ones' taps reach; the whole launch.
+// WgradBandKernel: a slice of so many positions; the whole launch.
 inline int WgradBandBytes(int positions) {
-    return ((positions + 16) * 64 + 1023) / 1024 * 1024;
+    return (positions * 64 + 1023) / 1024 * 1024;
 }
 // The stages, in whose place the sums of three taps are laid out at the end.
 __host__ __device__ inline int WgradBandData(const WgradBandArgs& a) {
