@@ -928,22 +928,6 @@ bool EncodeRows(CUtensorMap* m, const void* ptr, int rows, int kdim,
     return true;
 }
 
-int Pow2Cols(int n) {
-    int c = 32;
-    while (c < n) c *= 2;
-    return c;
-}
-
-// Largest divisor of c that is a multiple of 16 and at most 256.
-int PickBn(int c) {
-    for (int bn = 256; bn >= 16; bn -= 16)
-        if (c % bn == 0) return bn;
-    return 0;
-}
-
-constexpr int kSmemPerSm = 228 * 1024;
-constexpr int kSmemMax = 227 * 1024;
-
 // Dynamic shared memory for a launch: pads the request so that the CTAs an
 // SM can hold never ask for more than its 512 TMEM columns together.
 int ResidencySafeSmem(int smem, int tmem_cols) {
@@ -967,79 +951,6 @@ cudaError_t SetBandSmemAttr() {
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmemMax);
     return e;
-}
-
-// How a 3x3 convolution is cut into bands; tiles == 0: tap by tap instead.
-struct BandPlan {
-    int tiles = 0;    // per CTA
-    int bn = 0;
-    int rows = 0;     // image rows of a band's input box
-    int group = 0;    // k-blocks of a weight stage
-    int stages = 0;
-    int smem = 0;
-};
-
-// Tiles and output channels of a CTA (cold-L2 times of the network's layers, 32
-// images, against tap by tap: 32 -> 32 channels at 128^2 33 us, was 48; 64 -> 64
-// at 64^2 25, was 33; 128 -> 128 at 32^2 20, was 26), with fewer output channels
-// while the GPU is not full.  Above 128 input channels the
-// band fills the shared memory that the weights stream through (192 -> 64 at
-// 64^2 64 us, was 61; 384 -> 128 at 32^2 108, was 53).
-BandPlan PlanBand(int nimg, int H, int W, int cin, int cout, int bk,
-                  int sm_count) {
-    BandPlan p;
-    if (cin > 128) return p;
-    const int pitch = W + 2, step = W == 128 ? pitch : 128;
-    const int per_img = W == 128 ? H : ((H - 1) * pitch + W + 127) / 128;
-    const int chunks = (cin + bk - 1) / bk, nkb = 9 * chunks;
-    int bn = 128;
-    while (cout % bn != 0) bn -= 16;
-    int tiles = 1;
-    const auto ctas = [&] {
-        return (long long)nimg * ((per_img + tiles - 1) / tiles) * (cout / bn);
-    };
-    while (bn % 32 == 0 && bn > 32 && ctas() < sm_count) bn /= 2;
-    // Tiles of a CTA: its accumulators leave half of TMEM to another CTA.  An SM
-    // gets `per` CTAs, `per_sm` at a time, each such round costs about as much as
-    // a tile, and the fullest SM is the launch's time: 64 -> 64 at 64^2 (32
-    // images, 33 tiles each) 28 us with 1 tile, 25 with 2, 27 with 3; 32 -> 64
-    // 21, 19, 21 and with 4 17; 96 -> 32 at 128^2, 3 images, 19, 17, 12 and 15.
-    long long best = 0;
-    for (int most = std::min({4, bn <= 64 ? 4 : bn <= 96 ? 2 : 1, per_img});
-         tiles <= most; tiles++) {
-        const int rows = (W == 128 ? (tiles - 1) * step + 127
-                                   : pitch - 1 + (tiles - 1) * step + 127) /
-                             pitch + 3;
-        if (rows > 256) break;
-        const int chunk = BandChunkBytes(rows, pitch, bk);
-        const int kb_bytes = bn * bk * 2;
-        for (int per_sm = 2; per_sm >= 1; per_sm--) {
-            const int room = std::min(kSmemPerSm / per_sm - 2048, kSmemMax);
-            const int left = room - BandSmemBytes(chunks, chunk, 0, 0, bn, bk);
-            if (left < std::min(3, nkb) * (kb_bytes + 16)) continue;
-            const long long per = (ctas() + sm_count - 1) / sm_count;
-            const long long cost = (per + per_sm - 1) / per_sm + per * tiles;
-            if (p.tiles > 0 && cost > best) break;
-            best = cost;
-            // Waiting for a stage, committing it and forming its addresses
-            // cost about 500 cycles, as much as 12 MMAs: a stage holds enough
-            // k-blocks for 72, or all that fit (the other CTA of the SM runs
-            // meanwhile): 96 -> 32 at 128^2 90 us, with 32 98; 128 -> 128 at
-            // 32^2 18.5, with a third of what fits 20.2
-            const int mmas = tiles * (bk / 16);
-            p.group = std::min({nkb, (72 + mmas - 1) / mmas,
-                                left / (kb_bytes + 16)});
-            p.stages = std::min((nkb + p.group - 1) / p.group,
-                                left / (p.group * kb_bytes + 16));
-            p.tiles = tiles;
-            p.bn = bn;
-            p.rows = rows;
-            p.smem = BandSmemBytes(chunks, chunk, p.stages,
-                                   p.group * kb_bytes, bn, bk);
-            break;
-        }
-    }
-    return p;
 }
 
 bool LaunchConvBand(const View& x, const void* w, const BandPlan& p, int bk,
@@ -1127,7 +1038,7 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
         err = "fp32 output pixel stride must be a multiple of 4";
         return false;
     }
-    const int bk = x.c % 64 == 0 ? 64 : 32;
+    const int bk = ConvBk(x.c);
     const int bn = PickBn(y.c);
     if (bn == 0) {
         err = "output channels must be a multiple of 16";
@@ -1135,8 +1046,7 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
     }
     // 1x1 convolutions have no rows to keep in shared memory
     if (taps == 9) {
-        const BandPlan p =
-            PlanBand(x.nimg, x.h, x.w, x.c, y.c, bk, sm_count);
+        const BandPlan p = PlanBand(x.nimg, x.h, x.w, x.c, y.c, sm_count);
         if (p.tiles > 0)
             return LaunchConvBand(x, w, p, bk, bias, relu, y, y_f32, mask,
                                   stream, err_dev, err);
@@ -1154,9 +1064,7 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
     a.nkb = taps * ((x.c + bk - 1) / bk);
     a.cout = y.c;
     a.bn = bn;
-    a.stages = 4;
-    while (a.stages > 2 && ConvSmemBytes(bk, bn, a.stages) > 200 * 1024)
-        a.stages--;
+    a.stages = ConvStages(bk, bn);
     a.tmem_cols = Pow2Cols(bn);
     a.out = y.ptr;
     a.out_ps = y.ps;

@@ -49,11 +49,12 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include "conv_plan.h"
+
 namespace mplb {
 namespace nn {
 
 constexpr int kConvThreads = 128;
-constexpr int kTileM = 128;
 
 struct ConvArgs {
     int H, W;              // image size in pixels
@@ -191,27 +192,10 @@ __global__ void WgradKernel(const __grid_constant__ CUtensorMap ta,
                             const __grid_constant__ CUtensorMap tb,
                             WgradArgs a);
 
-// Shared memory a launch needs (stage buffers + 1 KiB alignment slack +
-// barriers).
-inline int ConvSmemBytes(int bk, int bn, int stages) {
-    return 1024 + stages * (kTileM * bk * 2 + bn * bk * 2) + 256;
-}
-// ConvBandKernel: a slice of a band's input - the last tile reads up to two
-// positions past its rows - and the whole launch.
-inline int BandChunkBytes(int rows, int pitch, int bk) {
-    return ((rows * pitch + 2) * bk * 2 + 1023) / 1024 * 1024;
-}
-inline int BandSmemBytes(int chunks, int chunk_bytes, int stages,
-                         int stage_bytes, int bn, int bk) {
-    return 1024 + chunks * chunk_bytes + stages * (stage_bytes + 16) +
-           bn * 4 + 8 * chunks + 64;
-}
+// Shared memory of the weight gradients' launches (the convolutions' and a
+// band's sizes are in conv_plan.h).
 inline int WgradSmemBytes(int b_atoms, int stages) {
     return 1024 + stages * ((2 + b_atoms) * 16384) + 256;
-}
-// WgradBandKernel: a slice of so many positions; the whole launch.
-inline int WgradBandBytes(int positions) {
-    return (positions * 64 + 1023) / 1024 * 1024;
 }
 // The stages, in whose place the sums of three taps are laid out at the end.
 __host__ __device__ inline int WgradBandData(const WgradBandArgs& a) {
