@@ -12,6 +12,7 @@
 // below into the lower channels of the concatenation buffer, two 3x3
 // convolutions with ReLU.  Output: 1x1 convolution to 16 fp32 channels of
 // which the first three are the normalised (rho, u, v).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -832,6 +833,61 @@ int* PrimErrWord() {
     return w;
 }
 
+// Start and end of the allocation that holds p; false if p is no memory that
+// the driver knows.
+bool AllocationOf(const void* p, const char** begin, const char** end) {
+    using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**,
+                            CUdeviceptr);
+    static const Fn get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPointByVersion(
+                            "cuPointerGetAttributes", &f, 12000,
+                            cudaEnableDefault, &q) == cudaSuccess &&
+                        q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Fn>(f) : nullptr;
+    }();
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* to[2] = {&start, &size};
+    if (get == nullptr ||
+        get(2, what, to, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS ||
+        size == 0) {
+        // memory without a range of its own: one byte at a time
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        *begin = static_cast<const char*>(p);
+        *end = *begin + 1;
+        return a.type != cudaMemoryTypeUnregistered;
+    }
+    *begin = reinterpret_cast<const char*>(start);
+    *end = *begin + size;
+    return true;
+}
+
+// Whether the samples `index` names, of `bytes` each from `base` on, are memory
+// the device can read.  A copy refuses a source that is not; a kernel's loads
+// would fault.
+bool Readable(const void* base, size_t bytes, const int* index, int n) {
+    const char* b = static_cast<const char*>(base);
+    const char *begin, *end;
+    if (!AllocationOf(b, &begin, &end)) return false;
+    const long long known = (end - b) / (long long)bytes;
+    for (int i = 0; i < n; i++) {
+        if (index[i] < known) continue;
+        const char* first = b + (size_t)index[i] * bytes;
+        const char* last = first + bytes - 1;
+        if (!AllocationOf(first, &begin, &end)) return false;
+        if (last >= end && !AllocationOf(last, &begin, &end)) return false;
+    }
+    return true;
+}
+
 int SmCount() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1089,6 +1145,9 @@ int mplbnn_loss_grad(mplbnn_net* net, const float* cond, const float* target,
         for (int i = 0; i < n; i++)
             if (index[i] < 0) return Fail(net, kInvalid, "negative index");
         const long long per = (long long)kGrid * kGrid * 3;
+        if (!Readable(cond, 3 * sizeof(float), index, n) ||
+            !Readable(target, per * sizeof(float), index, n))
+            return Fail(net, kInvalid, "index beyond the samples' memory");
         for (int i0 = 0; i0 < n; i0 += SampleIndex::kMost) {
             const int m = std::min(n - i0, (int)SampleIndex::kMost);
             SampleIndex at{};
