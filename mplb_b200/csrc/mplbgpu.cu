@@ -260,15 +260,29 @@ cudaError_t FillZeroF(mplbgpu_ctx* c, void* p, long long popstride) {
                                        popstride, Q, c->pc);
 }
 
+// cudaEventQuery(e) == cudaErrorNotReady.  A query may not be made while some
+// thread captures a stream in the global mode, this one's own capture included:
+// it would fail, and the capture with it.  The relaxed mode lifts that for this
+// call; the event is the context's own and never part of a capture (a caller who
+// captures the context's stream has asked for it, and then nothing is queried).
+bool StillRunning(cudaEvent_t e) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+    const bool running = cudaEventQuery(e) == cudaErrorNotReady;
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    (void)cudaGetLastError();   // not ready is no error
+    return running;
+}
+
 // Start and end of a step call's device time.  Step calls that follow one
 // another while the GPU is still on the last one start where it ended, so its
 // end event serves as the next one's start: each timed event holds the stream
-// for about 1.8 us, and a call a step is the reference's way of stepping.
-// Every other entry point waits for the stream or clears ev_chain.
+// for about 1.8 us, and a call a step is the reference's way of stepping.  (A
+// start event recorded then would take its time at that same end.)  Every other
+// entry point waits for the stream or clears ev_chain.
 int TimeStart(mplbgpu_ctx* ctx) {
     if (ctx->ev_chain && !ctx->stream_shared &&
-        cudaEventQuery(ctx->ev[ctx->ev_end]) == cudaErrorNotReady) {
-        (void)cudaGetLastError();   // not ready is no error
+        StillRunning(ctx->ev[ctx->ev_end])) {
         ctx->ev_start = ctx->ev_end;
     } else {
         ctx->ev_start = (ctx->ev_end + 1) % 3;
