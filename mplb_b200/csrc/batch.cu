@@ -14,7 +14,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <map>
 #include <string>
 #include <vector>
 
@@ -30,16 +29,6 @@ extern template struct mplb::BatchLaunch<double>;
 extern template struct mplb::BatchLaunch<float>;
 extern template struct mplb::BatchResidentLaunch<double>;
 extern template struct mplb::BatchResidentLaunch<float>;
-
-// Resident strips launched together: the same cluster size, slots and block.
-struct ResidentClass {
-    int halves, ranks, warps;
-    int max_steps;      // per launch
-    bool whole;         // every strip is a whole cavity
-    long long work;     // nodes computed per step
-    std::vector<ResidentItem> items;
-    int first = 0;      // of its items in the device list
-};
 
 struct mplbgpu_batch {
     int precision = MPLBGPU_FP32_SHIFTED;
@@ -159,153 +148,19 @@ int BuildTiles(mplbgpu_batch* b) {
     return MPLBGPU_OK;
 }
 
-// How the cavities of one side are held in shared memory.
-struct ResidentPlan {
-    int halves = 0, ranks = 1;
-    int strips = 1, overlap = 0;
-    double score = INFINITY;
-};
-
-// The best plan for cavities of side n when an SM has `load` nodes of the
-// active cavities to advance per step: the fewest SM cycles per node while
-// the GPU is full, the shortest step of one strip while it is not.  The
-// constants are measured on a B200: `fixed` is the part of a step that does
-// not shrink with its nodes (barrier, one pass' latency), `reload` the
-// reading and writing of a strip in steps of it, and the last table the share
-// of the SMs that clusters of that size can fill (a GPC's SMs are not always
-// a multiple of it).  Sweeps of every plan at sides 64-256 found none more than
-// 6 % faster than the one chosen here.
-ResidentPlan PlanResident(int n, bool f64, double load) {
-    static const int kRanks[] = {1, 2, 3, 4, 5, 6, 8, 9};
-    static const double kFill[] = {1.0, 1.0, 0.91, 0.89, 0.88, 0.89, 0.81,
-                                   0.91};
-    const double reload = f64 ? 1.3 : 2.5;
-    ResidentPlan best;
-    for (int halves = 0; halves < 3; halves++) {
-        const int cap = (f64 ? ResidentCap<double>() : ResidentCap<float>()) >>
-                        halves;
-        const double share = 1.0 / (1 << halves);
-        for (size_t r = 0; r < sizeof(kRanks) / sizeof(kRanks[0]); r++) {
-            const int ranks = kRanks[r];
-            const int most = ranks * (cap / n);   // rows of a strip
-            const double fixed = ranks > 1 ? 400 : 250;
-            auto consider = [&](int strips, int overlap, int rows) {
-                const double per_cta = (double)((rows + ranks - 1) / ranks) * n;
-                const double steps = strips > 1 ? overlap + 1 : 64;
-                const double cost = strips * ranks *
-                                    (per_cta + share * fixed) *
-                                    (1.0 + reload / steps) /
-                                    ((double)n * n * kFill[r]);
-                const double time = (per_cta + fixed) * (1.0 + reload / steps);
-                const double score =
-                    std::max(cost * load, time) + 0.1 * cost * load;
-                if (score >= best.score) return;
-                best.halves = halves;
-                best.ranks = ranks;
-                best.strips = strips;
-                best.overlap = overlap;
-                best.score = score;
-            };
-            if (most >= n) {
-                consider(1, 0, n);
-                continue;
-            }
-            for (int overlap : {3, 5, 7, 11, 15, 23}) {
-                const int inner = most - 2 * overlap;
-                if (inner < 1) break;
-                const int strips =
-                    std::max(2, (n - 2 * overlap + inner - 1) / inner);
-                const int valid = (n - 2 * overlap + strips - 1) / strips;
-                // the last strip takes what the others leave
-                if (n - overlap - (strips - 1) * valid < 1) continue;
-                consider(strips, overlap, valid + 2 * overlap);
-            }
-        }
-    }
-    return best;
-}
-
 // Resident strips of the active cavities, none if one does not fit.
 int BuildResident(mplbgpu_batch* b) {
     const bool f64 = b->precision == MPLBGPU_FP64;
-    b->resident.clear();
-    double nodes = 0;
-    for (int c : b->active) {
-        const double n = b->cav[c].n;
-        // rows of up to an eighth of the slots: larger cavities keep the
-        // tile launches (a strip would be mostly overlap)
-        if (n * 8 > (f64 ? ResidentCap<double>() : ResidentCap<float>()))
-            return MPLBGPU_OK;
-        nodes += n * n;
-    }
-    const int group = f64 ? ResidentGroup<double>() : ResidentGroup<float>();
     const long long unit = 128 / (f64 ? 8 : 4);
-    std::map<int, ResidentPlan> plans;
-    size_t count = 0;
-    for (int c : b->active) {
-        const int n = b->cav[c].n;
-        auto at = plans.find(n);
-        if (at == plans.end())
-            at = plans.emplace(n, PlanResident(n, f64, nodes / b->sms)).first;
-        const ResidentPlan& p = at->second;
-        const int valid = (n - 2 * p.overlap + p.strips - 1) / p.strips;
-        // the same block for all strips of a cavity: they read each other's
-        // rows of the launch before, so they stay in one class
-        const int tall = p.strips == 1 ? n : valid + 2 * p.overlap;
-        const int groups =
-            ((tall + p.ranks - 1) / p.ranks * n + group - 1) / group;
-        const int most = 24 >> p.halves;
-        const int passes = (groups + most - 1) / most;
-        const int warps = std::max(2, (groups + passes - 1) / passes);
-        const int max_steps = p.strips == 1 ? 128 : p.overlap + 1;
-        for (int j = 0; j < p.strips; j++) {
-            ResidentItem it{};
-            it.cav = c;
-            it.n = n;
-            it.base = (int)(b->hcav[c].base / unit);
-            it.whole = p.strips == 1;
-            const int v0 = j == 0 ? 0 : p.overlap + j * valid;
-            const int v1 = j + 1 == p.strips ? n : p.overlap + (j + 1) * valid;
-            it.row0 = std::max(0, v0 - p.overlap);
-            it.rows = std::min(n, v1 + p.overlap) - it.row0;
-            it.vrow0 = v0 - it.row0;
-            it.vrows = v1 - v0;
-            it.rows_per_cta = (it.rows + p.ranks - 1) / p.ranks;
-            ResidentClass* cls = nullptr;
-            for (ResidentClass& k : b->resident)
-                if (k.halves == p.halves && k.ranks == p.ranks &&
-                    k.warps == warps && k.max_steps == max_steps)
-                    cls = &k;
-            if (!cls) {
-                ResidentClass k{};
-                k.halves = p.halves;
-                k.ranks = p.ranks;
-                k.warps = warps;
-                k.max_steps = max_steps;
-                k.whole = it.whole != 0;
-                b->resident.push_back(k);
-                cls = &b->resident.back();
-            }
-            cls->items.push_back(it);
-            cls->work += (long long)it.rows * n;
-            count++;
-        }
+    std::vector<int> sides, base;
+    for (size_t c = 0; c < b->cav.size(); c++) {
+        sides.push_back(b->cav[c].n);
+        base.push_back((int)(b->hcav[c].base / unit));
     }
-    // the longest class first; within a class the longest strips first
-    std::sort(b->resident.begin(), b->resident.end(),
-              [](const ResidentClass& x, const ResidentClass& y) {
-                  return x.work > y.work;
-              });
+    b->resident = PlanStrips(b->active, sides, base, f64, b->sms);
     std::vector<ResidentItem> all;
-    for (ResidentClass& k : b->resident) {
-        std::stable_sort(k.items.begin(), k.items.end(),
-                         [](const ResidentItem& x, const ResidentItem& y) {
-                             return x.rows_per_cta * x.n >
-                                    y.rows_per_cta * y.n;
-                         });
-        k.first = (int)all.size();
+    for (const ResidentClass& k : b->resident)
         all.insert(all.end(), k.items.begin(), k.items.end());
-    }
     for (size_t k = 0; k + 1 < b->resident.size() && k < mplbgpu_batch::kSides;
          k++) {
         if (!b->fork)
@@ -315,6 +170,7 @@ int BuildResident(mplbgpu_batch* b) {
         if (!b->join[k])
             BCK(cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming));
     }
+    const size_t count = all.size();
     if (count > b->items_cap) {
         BCK(cudaFree(b->items));
         b->items = nullptr;

@@ -36,26 +36,9 @@
 #pragma once
 
 #include "batch_kernels.cuh"
+#include "batch_plan.h"
 
 namespace mplb {
-
-// A strip of a cavity: rows [row0, row0 + rows) are computed, rows
-// [vrow0, vrow0 + vrows) (counted from row0) are stored.
-struct ResidentItem {
-    int cav;
-    int n;
-    int base;        // element offset of the cavity, in 128-byte units
-    int row0, rows;
-    int vrow0, vrows;
-    int rows_per_cta;
-    int whole;       // the strip is the whole cavity: stored where it is read
-};
-
-// Nodes whose slots fill an SM's shared memory (230,400 bytes).
-template <typename T>
-__host__ __device__ constexpr int ResidentCap() {
-    return sizeof(T) == 4 ? 6400 : 3200;
-}
 
 __device__ __forceinline__ uint32_t ClusterRank() {
     uint32_t r;
@@ -308,10 +291,9 @@ __device__ __forceinline__ void ResidentNodes(const BatchDev& bd,
     }
 }
 
-// Nodes a thread advances at once, and so the nodes of a warp.
 template <typename T>
 __host__ __device__ constexpr int ResidentGroup() {
-    return sizeof(T) == 4 ? 64 : 32;
+    return sizeof(T) == 4 ? kResidentGroup32 : kResidentGroup64;
 }
 
 // One step over the CTA's nodes.  Only steps that reach into another CTA's
@@ -342,16 +324,12 @@ __device__ __forceinline__ void ResidentStep(const BatchDev& bd,
     }
 }
 
-// Threads of a CTA, at most: 24 warps of 80 registers share an SM, whose slots
-// one, two or four CTAs fill.
-template <typename T, int CAP>
-__host__ __device__ constexpr int ResidentMaxThreads() {
-    return CAP == ResidentCap<T>() ? 768 : 384 * 2 * CAP / ResidentCap<T>();
-}
-
-template <typename T, int CAP>
-__global__ void __launch_bounds__(ResidentMaxThreads<T, CAP>(),
-                                  ResidentCap<T>() / CAP)
+// 24 warps of 80 registers share an SM, whose slots one, two or four CTAs fill
+// (side 24, crowded: FP32 185 G, FP64 97 G; three CTAs of 18 warps, which is
+// what fits when a quarter's slots leave no room for the CTAs' own 1 KB: 166 G
+// and 91 G).
+template <typename T, int HALVES, int CAP>
+__global__ void __launch_bounds__(768 >> HALVES, 1 << HALVES)
     BatchResidentKernel(BatchDev bd, PhysConst pc,
                         const ResidentItem* __restrict__ items, int steps,
                         int macro, const T* src, T* dst) {
@@ -423,24 +401,24 @@ struct BatchResidentLaunch {
                            cudaStream_t s, const BatchDev& bd,
                            const PhysConst& pc, const ResidentItem* items,
                            int steps, bool macro, const T* src, T* dst) {
-        constexpr int kCap = ResidentCap<T>();
-        return halves == 0 ? RunCap<kCap>(ranks, warps, nitems, s, bd, pc,
-                                          items, steps, macro, src, dst)
+        return halves == 0 ? RunForm<0>(ranks, warps, nitems, s, bd, pc, items,
+                                        steps, macro, src, dst)
                : halves == 1
-                   ? RunCap<kCap / 2>(ranks, warps, nitems, s, bd, pc, items,
-                                      steps, macro, src, dst)
-                   : RunCap<kCap / 4>(ranks, warps, nitems, s, bd, pc, items,
-                                      steps, macro, src, dst);
+                   ? RunForm<1>(ranks, warps, nitems, s, bd, pc, items, steps,
+                                macro, src, dst)
+                   : RunForm<2>(ranks, warps, nitems, s, bd, pc, items, steps,
+                                macro, src, dst);
     }
 
   private:
-    template <int CAP>
-    static cudaError_t RunCap(int ranks, int warps, int nitems, cudaStream_t s,
-                              const BatchDev& bd, const PhysConst& pc,
-                              const ResidentItem* items, int steps, bool macro,
-                              const T* src, T* dst) {
-        auto* kernel = BatchResidentKernel<T, CAP>;
-        constexpr int kSmem = 9 * CAP * (int)sizeof(T);
+    template <int HALVES>
+    static cudaError_t RunForm(int ranks, int warps, int nitems,
+                               cudaStream_t s, const BatchDev& bd,
+                               const PhysConst& pc, const ResidentItem* items,
+                               int steps, bool macro, const T* src, T* dst) {
+        constexpr int kCap = ResidentSlots(sizeof(T) == 8, HALVES);
+        auto* kernel = BatchResidentKernel<T, HALVES, kCap>;
+        constexpr int kSmem = ResidentSmem(sizeof(T) == 8, HALVES);
         cudaError_t e = cudaFuncSetAttribute(
             kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
         if (e == cudaSuccess && ranks > 8)
