@@ -73,6 +73,7 @@ struct mplbgpu_batch {
     ResidentItem* items = nullptr;
     size_t items_cap = 0;
     int sms = 1;
+    ResidentHeld held;
     static constexpr int kSides = 5;   // side streams of the classes, made
                                        // when a plan first needs them
     cudaStream_t side[kSides] = {};
@@ -157,7 +158,7 @@ int BuildResident(mplbgpu_batch* b) {
         sides.push_back(b->cav[c].n);
         base.push_back((int)(b->hcav[c].base / unit));
     }
-    b->resident = PlanStrips(b->active, sides, base, f64, b->sms);
+    b->resident = PlanStrips(b->active, sides, base, f64, b->sms, b->held);
     std::vector<ResidentItem> all;
     for (const ResidentClass& k : b->resident)
         all.insert(all.end(), k.items.begin(), k.items.end());
@@ -204,6 +205,7 @@ int AdvanceResident(mplbgpu_batch* b, long long nsteps, bool macro_last) {
             BCK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
     }
     double busy[mplbgpu_batch::kSides + 1] = {};
+    cudaError_t failed = cudaSuccess;
     for (const ResidentClass& k : b->resident) {
         // to the stream that is free first: a class takes its share of the
         // GPU's work, at least the time of its longest strip
@@ -222,15 +224,19 @@ int AdvanceResident(mplbgpu_batch* b, long long nsteps, bool macro_last) {
                 b->items + k.first, n, macro_last && l + 1 == count,
                 pop[k.whole ? 0 : (l & 1)], pop[k.whole ? 0 : 1 - (l & 1)]);
             b->launches++;
-            if (e != cudaSuccess)
-                return BErr(b, MPLBGPU_ERR_CUDA,
-                            std::string("resident launch: ") +
-                                cudaGetErrorString(e));
+            if (e != cudaSuccess && failed == cudaSuccess) failed = e;
         }
     }
+    // also behind a launch that failed: nothing of the batch's runs on
     for (int k = 0; k < lanes - 1; k++) {
         BCK(cudaEventRecord(b->join[k], b->side[k]));
         BCK(cudaStreamWaitEvent(b->stream, b->join[k], 0));
+    }
+    if (failed != cudaSuccess) {
+        b->initialised = false;   // some strips are steps ahead of others
+        return BErr(b, MPLBGPU_ERR_CUDA,
+                    std::string("resident launch: ") +
+                        cudaGetErrorString(failed));
     }
     b->pc.seed += (uint32_t)nsteps;
     return MPLBGPU_OK;
@@ -529,6 +535,12 @@ mplbgpu_status mplbgpu_batch_create(const mplbgpu_cavity* cavities, int ncav,
     int dev = 0;
     CRE(cudaGetDevice(&dev));
     CRE(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
+    for (int h = 0; h < 3; h++)
+        for (int r = 0; r < kNumResidentRanks; r++)
+            b->held.at[h][r] =
+                precision == MPLBGPU_FP64
+                    ? BatchResidentLaunch<double>::Held(h, kResidentRanks[r])
+                    : BatchResidentLaunch<float>::Held(h, kResidentRanks[r]);
     CRE(cudaMalloc(&b->dcav, ncav * sizeof(BatchCav)));
     CRE(cudaMemcpy(b->dcav, b->hcav.data(), ncav * sizeof(BatchCav),
                    cudaMemcpyHostToDevice));

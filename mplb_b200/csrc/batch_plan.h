@@ -58,7 +58,17 @@ struct ResidentClass {
     int first = 0;      // of its items in the list of all
 };
 
-// How the cavities of one side are held in shared memory.
+// Cluster sizes of the plans, and which of them, in which form, the device can
+// hold at all: part of a GPU (fewer SMs in its GPCs, less shared memory left) may
+// have no place for some that a whole B200 has.
+constexpr int kResidentRanks[] = {1, 2, 3, 4, 5, 6, 8, 9};
+constexpr int kNumResidentRanks = 8;
+struct ResidentHeld {
+    bool at[3][kNumResidentRanks] = {};   // [halves][index of the ranks]
+};
+
+// How the cavities of one side are held in shared memory; score infinite: not
+// at all.
 struct ResidentPlan {
     int halves = 0, ranks = 1;
     int strips = 1, overlap = 0;
@@ -74,8 +84,8 @@ struct ResidentPlan {
 // of the SMs that clusters of that size can fill (a GPC's SMs are not always
 // a multiple of it).  Sweeps of every plan at sides 64-256 found none more than
 // 6 % faster than the one chosen here.
-inline ResidentPlan PlanResident(int n, bool f64, double load) {
-    static const int kRanks[] = {1, 2, 3, 4, 5, 6, 8, 9};
+inline ResidentPlan PlanResident(int n, bool f64, double load,
+                                 const ResidentHeld& held) {
     static const double kFill[] = {1.0, 1.0, 0.91, 0.89, 0.88, 0.89, 0.81,
                                    0.91};
     const double reload = f64 ? 1.3 : 2.5;
@@ -83,8 +93,9 @@ inline ResidentPlan PlanResident(int n, bool f64, double load) {
     for (int halves = 0; halves < 3; halves++) {
         const int cap = ResidentSlots(f64, halves);
         const double share = 1.0 / (1 << halves);
-        for (size_t r = 0; r < sizeof(kRanks) / sizeof(kRanks[0]); r++) {
-            const int ranks = kRanks[r];
+        for (int r = 0; r < kNumResidentRanks; r++) {
+            if (!held.at[halves][r]) continue;
+            const int ranks = kResidentRanks[r];
             const int most = ranks * (cap / n);   // rows of a strip
             const double fixed = ranks > 1 ? 400 : 250;
             auto consider = [&](int strips, int overlap, int rows) {
@@ -125,11 +136,13 @@ inline ResidentPlan PlanResident(int n, bool f64, double load) {
 
 // Resident strips of the cavities `active` of the sides `sides` (base: their
 // element offsets in 128-byte units) on a GPU of `sms` SMs, the longest class
-// first, the longest strips of a class first; none if a cavity does not fit.
+// first, the longest strips of a class first; none if a cavity does not fit in
+// what the device holds.
 inline std::vector<ResidentClass> PlanStrips(const std::vector<int>& active,
                                              const std::vector<int>& sides,
                                              const std::vector<int>& base,
-                                             bool f64, int sms) {
+                                             bool f64, int sms,
+                                             const ResidentHeld& held) {
     std::vector<ResidentClass> classes;
     double nodes = 0;
     for (int c : active) {
@@ -143,8 +156,10 @@ inline std::vector<ResidentClass> PlanStrips(const std::vector<int>& active,
         const int n = sides[c];
         auto at = plans.find(n);
         if (at == plans.end())
-            at = plans.emplace(n, PlanResident(n, f64, nodes / sms)).first;
+            at = plans.emplace(n, PlanResident(n, f64, nodes / sms, held))
+                     .first;
         const ResidentPlan& p = at->second;
+        if (std::isinf(p.score)) return {};
         const int valid = (n - 2 * p.overlap + p.strips - 1) / p.strips;
         // the same block for all strips of a cavity: they read each other's
         // rows of the launch before, so they stay in one class

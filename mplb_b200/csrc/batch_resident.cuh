@@ -401,44 +401,60 @@ struct BatchResidentLaunch {
                            cudaStream_t s, const BatchDev& bd,
                            const PhysConst& pc, const ResidentItem* items,
                            int steps, bool macro, const T* src, T* dst) {
-        return halves == 0 ? RunForm<0>(ranks, warps, nitems, s, bd, pc, items,
-                                        steps, macro, src, dst)
-               : halves == 1
-                   ? RunForm<1>(ranks, warps, nitems, s, bd, pc, items, steps,
-                                macro, src, dst)
-                   : RunForm<2>(ranks, warps, nitems, s, bd, pc, items, steps,
-                                macro, src, dst);
+        Config c(halves, ranks, warps, nitems, s);
+        cudaError_t e = Prepare(halves, ranks);
+        if (e != cudaSuccess) return e;
+        return cudaLaunchKernelEx(&c.cfg, Kernel(halves), bd, pc, items, steps,
+                                  macro ? 1 : 0, src, dst);
+    }
+    // Whether the device can hold a cluster of `ranks` such CTAs.
+    static bool Held(int halves, int ranks) {
+        Config c(halves, ranks, 24 >> halves, 1, nullptr);
+        int clusters = 0;
+        if (Prepare(halves, ranks) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, Kernel(halves),
+                                           &c.cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        return clusters > 0;
     }
 
   private:
-    template <int HALVES>
-    static cudaError_t RunForm(int ranks, int warps, int nitems,
-                               cudaStream_t s, const BatchDev& bd,
-                               const PhysConst& pc, const ResidentItem* items,
-                               int steps, bool macro, const T* src, T* dst) {
-        constexpr int kCap = ResidentSlots(sizeof(T) == 8, HALVES);
-        auto* kernel = BatchResidentKernel<T, HALVES, kCap>;
-        constexpr int kSmem = ResidentSmem(sizeof(T) == 8, HALVES);
+    using KernelFn = void (*)(BatchDev, PhysConst, const ResidentItem*, int,
+                              int, const T*, T*);
+    static constexpr bool kF64 = sizeof(T) == 8;
+
+    struct Config {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr{};
+        Config(int halves, int ranks, int warps, int nitems, cudaStream_t s) {
+            cfg.gridDim = dim3((unsigned)nitems * (unsigned)ranks);
+            cfg.blockDim = dim3((unsigned)warps * 32u);
+            cfg.dynamicSmemBytes = ResidentSmem(kF64, halves);
+            cfg.stream = s;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)ranks;
+            attr.val.clusterDim.y = 1;
+            attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+        }
+    };
+    static KernelFn Kernel(int halves) {
+        return halves == 0   ? BatchResidentKernel<T, 0, ResidentSlots(kF64, 0)>
+               : halves == 1 ? BatchResidentKernel<T, 1, ResidentSlots(kF64, 1)>
+                             : BatchResidentKernel<T, 2, ResidentSlots(kF64, 2)>;
+    }
+    static cudaError_t Prepare(int halves, int ranks) {
         cudaError_t e = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+            Kernel(halves), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            ResidentSmem(kF64, halves));
         if (e == cudaSuccess && ranks > 8)
             e = cudaFuncSetAttribute(
-                kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)nitems * (unsigned)ranks);
-        cfg.blockDim = dim3((unsigned)warps * 32u);
-        cfg.dynamicSmemBytes = kSmem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)ranks;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kernel, bd, pc, items, steps,
-                                  macro ? 1 : 0, src, dst);
+                Kernel(halves), cudaFuncAttributeNonPortableClusterSizeAllowed,
+                1);
+        return e;
     }
 };
 

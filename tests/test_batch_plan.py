@@ -22,10 +22,19 @@ int main() {
             printf("%d %d\n", ResidentSlots(f64, n), ResidentSmem(f64, n));
             continue;
         }
+        ResidentHeld held;
+        for (int h = 0; h < 3; h++)
+            for (int r = 0; r < kNumResidentRanks; r++)
+                held.at[h][r] = !strcmp(what, "plan") ||
+                                (!strcmp(what, "portable") &&
+                                 kResidentRanks[r] <= 8) ||
+                                (!strcmp(what, "single") && h > 0 &&
+                                 kResidentRanks[r] == 1);
         std::vector<int> active, sides(count, n), base(count, 0);
         for (int c = 0; c < count; c++) active.push_back(c);
         printf("%d", ResidentMaxSide(f64));
-        for (const ResidentClass& k : PlanStrips(active, sides, base, f64, 148))
+        for (const ResidentClass& k : PlanStrips(active, sides, base, f64, 148,
+                                               held))
             for (const ResidentItem& i : k.items)
                 if (i.cav == 0)
                     printf(" %d %d %d %d %d %d %d %d", k.halves, k.ranks,
@@ -41,7 +50,7 @@ int main() {
 def ask(tmp_path_factory):
     d = tmp_path_factory.mktemp("plan")
     (d / "ask.cpp").write_text(SOURCE)
-    subprocess.run(["g++", "-O1", "-std=c++17", "-I", build.CSRC, "-o",
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", build.CSRC, "-o",
                     d / "ask", d / "ask.cpp"], check=True)
 
     def run(lines):
@@ -62,21 +71,29 @@ def test_the_ctas_of_a_form_share_an_sm(ask, f64):
 
 
 @pytest.mark.parametrize("f64", [0, 1])
+@pytest.mark.parametrize("what, most_ranks, least_halves", [
+    ("plan", 9, 0), ("portable", 8, 0), ("single", 1, 1)])
 @pytest.mark.parametrize("count", [1, 30, 3000])
-def test_strips_cover_every_side(ask, f64, count):
+def test_strips_cover_every_side(ask, f64, count, what, most_ranks,
+                                 least_halves):
+    """On a whole GPU, and on one that cannot hold clusters beyond the portable
+    size, or none and no CTA of a whole SM's slots."""
     largest = 400 if f64 else 800
     slots = [s for s, _ in ask([f"form {f64} {h} 0" for h in range(3)])]
-    sides = list(range(3, largest + 1))
-    got = ask([f"plan {f64} {n} {count}" for n in sides])
+    sides = list(range(3, largest + 1, 1 if what == "plan" else 7))
+    got = ask([f"{what} {f64} {n} {count}" for n in sides])
     for n, (most, *flat) in zip(sides, got):
         assert most == largest
         strips = sorted((flat[i:i + 8] for i in range(0, len(flat), 8)),
                         key=lambda s: s[4])
-        assert strips, n
+        if not strips:      # too few rows of slots for any overlap
+            assert what == "single" and slots[1] // n < 2 * 3 + 1
+            continue
         row = 0
         for halves, ranks, warps, steps, row0, rows, vrow0, vrows in strips:
             assert -(-rows // ranks) * n <= slots[halves]
             assert 2 <= warps <= 24 >> halves
+            assert ranks <= most_ranks and halves >= least_halves
             assert row0 + vrow0 == row and vrows > 0
             row += vrows
             # a cut edge's wrong values travel a row a step after the first
@@ -90,3 +107,7 @@ def test_strips_cover_every_side(ask, f64, count):
 
 def test_a_side_beyond_the_slots_has_no_strips(ask):
     assert ask(["plan 0 801 2", "plan 1 401 2"]) == [[800], [400]]
+
+
+def test_a_device_that_holds_none_has_no_strips(ask):
+    assert ask(["none 0 64 2", "none 1 64 2"]) == [[800], [400]]
