@@ -27,7 +27,7 @@ HEADERS = [os.path.join(CSRC, h) for h in ("kernels.cuh", "lattice.h",
                                             "launch_impl.cuh", "swap.cuh",
                                             "double_step.cuh",
                                             "batch_kernels.cuh",
-                                            "batch_plan.h",
+                                            "batch_plan.h", "batch_launch.h",
                                             "batch_resident.cuh", "tma.cuh",
                                             "nn/umma.cuh", "nn/conv.cuh",
                                             "nn/conv_host.h", "nn/conv_plan.h",

@@ -18,17 +18,10 @@
 #include <vector>
 
 #include "../../include/mplbgpu.h"
-#include "batch_resident.cuh"
+#include "batch_launch.h"
 #include "lattice.h"
 
 using namespace mplb;
-
-// The launchers are instantiated in kernels_f64.cu / kernels_lp.cu with the
-// floating-point contraction rules of their forms.
-extern template struct mplb::BatchLaunch<double>;
-extern template struct mplb::BatchLaunch<float>;
-extern template struct mplb::BatchResidentLaunch<double>;
-extern template struct mplb::BatchResidentLaunch<float>;
 
 struct mplbgpu_batch {
     int precision = MPLBGPU_FP32_SHIFTED;

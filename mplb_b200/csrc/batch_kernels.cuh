@@ -13,42 +13,9 @@
 // base + p n^2 + k, structure of arrays per cavity, no halo.
 #pragma once
 
-#include "kernels.cuh"
+#include "batch_launch.h"
 
 namespace mplb {
-
-struct BatchCav {
-    long long base;    // element offset of the cavity in a population array
-    long long mbase;   // offset of its nodes in the macro arrays
-    int n;             // nodes per side
-    int pad;
-    double omc;        // 1 - omega of this cavity
-    double dt;         // MPLB time step (residual normalisation)
-    float omcf;
-    float ninv;        // 1 / n (row of node k: (k + 1/2) / n rounded down)
-    double lidb[9];    // 2 w_i (c_i . u_lid) for populations bounced at the lid
-    float lidbf[9];
-};
-
-struct BatchDev {
-    const BatchCav* cavs;
-    // active tiles: (cavity, first node, nodes per side, element offset of
-    // the cavity in 128-byte units), so a tile's population addresses wait
-    // on the tile's own load alone and the cavity's constants load beside
-    // the populations
-    const int4* tiles;
-    const int* ntiles;      // number of active tiles (device word)
-    int tile_nodes;         // nodes per tile
-    double* macro[3];       // rho, u, v of every cavity, packed
-    double* macro_old[3];
-};
-
-struct GridSync {           // bounded grid-wide barrier state
-    unsigned* count;
-    unsigned* gen;
-    int* err;               // set to 1 when a wait gives up
-    long long limit;        // polls before giving up
-};
 
 // Every population value is read once and written once per step, so the
 // batch's loads and stores take the streaming (evict-first) cache hint and
@@ -202,18 +169,6 @@ __device__ __forceinline__ void BatchNodeGroup(const BatchDev& bd,
     }
 }
 
-#ifndef MPLB_BATCH_GROUP
-#define MPLB_BATCH_GROUP 2
-#endif
-
-// Nodes per thread of the step kernels (threads per CTA = tile nodes / this):
-// MPLB_BATCH_GROUP in the FP32 form, one in FP64.
-template <typename T>
-__host__ __device__ constexpr int BatchNodesPerThread() {
-    return sizeof(T) < 8 ? MPLB_BATCH_GROUP : 1;
-}
-
-
 template <typename T, bool MACRO>
 __device__ __forceinline__ void BatchSweep(const BatchDev& bd,
                                            const PhysConst& pc, int nt,
@@ -310,19 +265,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Per active tile: sum (q - q_old)^2 and sum q^2 of rho, u, v; q_old <- q.
-__global__ void BatchResidualPartialKernel(BatchDev bd,
-                                           double* __restrict__ part);
-
-// Per active cavity c (CTA c): sums its tiles' partials in order and writes
-// max_q [sum (q - q_old)^2 / sum q^2] / (check_period dt) (the reference's
-// CalcResidualError + GetMaximumResidual on one cavity).
-__global__ void BatchResidualFinalKernel(BatchDev bd,
-                                         const double* __restrict__ part,
-                                         const int4* __restrict__ ranges,
-                                         int ncav, int check_period,
-                                         double* __restrict__ res);
-
 // Initial state: f^0 = feq(rho, u, v) from the packed macro fields
 // (KerInitialiseBGK2nd), then g^0 = collision of f^0 with its own moments,
 // as the first StreamCollision would do, into `a`.
@@ -371,47 +313,46 @@ __global__ void BatchInitKernel(BatchDev bd, PhysConst pc,
     }
 }
 
-}  // namespace mplb
-
-namespace mplb {
-
-// Host launchers, instantiated with the FP64 and the FP32 forms.
 template <typename T>
-struct BatchLaunch {
-    static cudaError_t Step(bool macro, int grid, int threads, cudaStream_t s,
-                            const BatchDev& bd, const PhysConst& pc, int nt,
-                            const T* src, T* dst) {
-        if (macro)
-            BatchStepKernel<T, true><<<grid, threads, 0, s>>>(bd, pc, nt, src,
-                                                              dst);
-        else
-            BatchStepKernel<T, false><<<grid, threads, 0, s>>>(bd, pc, nt, src,
-                                                               dst);
-        return cudaGetLastError();
-    }
-    static cudaError_t Persistent(int grid, int threads, cudaStream_t s,
-                                  const BatchDev& bd, const PhysConst& pc,
-                                  T* a, T* b, int nsteps, int macro_last,
-                                  const GridSync& gs) {
-        BatchDev bdv = bd;
-        PhysConst pcv = pc;
-        GridSync gsv = gs;
-        void* args[] = {&bdv, &pcv, &a, &b, &nsteps, &macro_last, &gsv};
-        return cudaLaunchCooperativeKernel(
-            (const void*)BatchPersistentKernel<T>, dim3(grid), dim3(threads),
-            args, 0, s);
-    }
-    static cudaError_t MaxCoResident(int threads, int* per_sm) {
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            per_sm, (const void*)BatchPersistentKernel<T>, threads, 0);
-    }
-    static cudaError_t Init(int grid, int threads, cudaStream_t s,
-                            const BatchDev& bd, const PhysConst& pc,
-                            const int4* alltiles, int ntiles, T* a) {
-        BatchInitKernel<T><<<grid, threads, 0, s>>>(bd, pc, alltiles, ntiles,
-                                                    a);
-        return cudaGetLastError();
-    }
-};
+cudaError_t BatchLaunch<T>::Step(bool macro, int grid, int threads,
+                                 cudaStream_t s, const BatchDev& bd,
+                                 const PhysConst& pc, int nt, const T* src,
+                                 T* dst) {
+    if (macro)
+        BatchStepKernel<T, true><<<grid, threads, 0, s>>>(bd, pc, nt, src,
+                                                          dst);
+    else
+        BatchStepKernel<T, false><<<grid, threads, 0, s>>>(bd, pc, nt, src,
+                                                           dst);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t BatchLaunch<T>::Persistent(int grid, int threads, cudaStream_t s,
+                                       const BatchDev& bd, const PhysConst& pc,
+                                       T* a, T* b, int nsteps, int macro_last,
+                                       const GridSync& gs) {
+    BatchDev bdv = bd;
+    PhysConst pcv = pc;
+    GridSync gsv = gs;
+    void* args[] = {&bdv, &pcv, &a, &b, &nsteps, &macro_last, &gsv};
+    return cudaLaunchCooperativeKernel(
+        (const void*)BatchPersistentKernel<T>, dim3(grid), dim3(threads), args,
+        0, s);
+}
+
+template <typename T>
+cudaError_t BatchLaunch<T>::MaxCoResident(int threads, int* per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        per_sm, (const void*)BatchPersistentKernel<T>, threads, 0);
+}
+
+template <typename T>
+cudaError_t BatchLaunch<T>::Init(int grid, int threads, cudaStream_t s,
+                                 const BatchDev& bd, const PhysConst& pc,
+                                 const int4* alltiles, int ntiles, T* a) {
+    BatchInitKernel<T><<<grid, threads, 0, s>>>(bd, pc, alltiles, ntiles, a);
+    return cudaGetLastError();
+}
 
 }  // namespace mplb

@@ -36,7 +36,6 @@
 #pragma once
 
 #include "batch_kernels.cuh"
-#include "batch_plan.h"
 
 namespace mplb {
 
@@ -393,69 +392,73 @@ __global__ void __launch_bounds__(768 >> HALVES, 1 << HALVES)
     barrier();   // no CTA leaves while another may read its slots
 }
 
-// Host launcher, instantiated with the FP64 and the FP32 forms.
 template <typename T>
-struct BatchResidentLaunch {
-    // `halves`: the CTAs' slots fill 1 / 2^halves of an SM.
-    static cudaError_t Run(int halves, int ranks, int warps, int nitems,
-                           cudaStream_t s, const BatchDev& bd,
-                           const PhysConst& pc, const ResidentItem* items,
-                           int steps, bool macro, const T* src, T* dst) {
-        Config c(halves, ranks, warps, nitems, s);
-        cudaError_t e = Prepare(halves, ranks);
-        if (e != cudaSuccess) return e;
-        return cudaLaunchKernelEx(&c.cfg, Kernel(halves), bd, pc, items, steps,
-                                  macro ? 1 : 0, src, dst);
-    }
-    // Whether the device can hold a cluster of `ranks` such CTAs.
-    static bool Held(int halves, int ranks) {
-        Config c(halves, ranks, 24 >> halves, 1, nullptr);
-        int clusters = 0;
-        if (Prepare(halves, ranks) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&clusters, Kernel(halves),
-                                           &c.cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return false;
-        }
-        return clusters > 0;
-    }
-
-  private:
-    using KernelFn = void (*)(BatchDev, PhysConst, const ResidentItem*, int,
-                              int, const T*, T*);
-    static constexpr bool kF64 = sizeof(T) == 8;
-
-    struct Config {
-        cudaLaunchConfig_t cfg{};
-        cudaLaunchAttribute attr{};
-        Config(int halves, int ranks, int warps, int nitems, cudaStream_t s) {
-            cfg.gridDim = dim3((unsigned)nitems * (unsigned)ranks);
-            cfg.blockDim = dim3((unsigned)warps * 32u);
-            cfg.dynamicSmemBytes = ResidentSmem(kF64, halves);
-            cfg.stream = s;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = (unsigned)ranks;
-            attr.val.clusterDim.y = 1;
-            attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-        }
-    };
-    static KernelFn Kernel(int halves) {
-        return halves == 0   ? BatchResidentKernel<T, 0, ResidentSlots(kF64, 0)>
-               : halves == 1 ? BatchResidentKernel<T, 1, ResidentSlots(kF64, 1)>
-                             : BatchResidentKernel<T, 2, ResidentSlots(kF64, 2)>;
-    }
-    static cudaError_t Prepare(int halves, int ranks) {
-        cudaError_t e = cudaFuncSetAttribute(
-            Kernel(halves), cudaFuncAttributeMaxDynamicSharedMemorySize,
-            ResidentSmem(kF64, halves));
-        if (e == cudaSuccess && ranks > 8)
-            e = cudaFuncSetAttribute(
-                Kernel(halves), cudaFuncAttributeNonPortableClusterSizeAllowed,
-                1);
-        return e;
+using ResidentKernelFn = void (*)(BatchDev, PhysConst, const ResidentItem*, int,
+                                  int, const T*, T*);
+template <typename T>
+ResidentKernelFn<T> ResidentKernelOf(int halves) {
+    constexpr bool kF64 = sizeof(T) == 8;
+    return halves == 0   ? BatchResidentKernel<T, 0, ResidentSlots(kF64, 0)>
+           : halves == 1 ? BatchResidentKernel<T, 1, ResidentSlots(kF64, 1)>
+                         : BatchResidentKernel<T, 2, ResidentSlots(kF64, 2)>;
+}
+template <typename T>
+cudaError_t PrepareResident(int halves, int ranks) {
+    cudaError_t e = cudaFuncSetAttribute(
+        ResidentKernelOf<T>(halves),
+        cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ResidentSmem(sizeof(T) == 8, halves));
+    if (e == cudaSuccess && ranks > 8)
+        e = cudaFuncSetAttribute(ResidentKernelOf<T>(halves),
+                                 cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                 1);
+    return e;
+}
+struct ResidentConfig {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    ResidentConfig(int smem, int ranks, int warps, int nitems,
+                   cudaStream_t s) {
+        cfg.gridDim = dim3((unsigned)nitems * (unsigned)ranks);
+        cfg.blockDim = dim3((unsigned)warps * 32u);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)ranks;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
     }
 };
+
+template <typename T>
+cudaError_t BatchResidentLaunch<T>::Run(int halves, int ranks, int warps,
+                                        int nitems, cudaStream_t s,
+                                        const BatchDev& bd,
+                                        const PhysConst& pc,
+                                        const ResidentItem* items, int steps,
+                                        bool macro, const T* src, T* dst) {
+    ResidentConfig c(ResidentSmem(sizeof(T) == 8, halves), ranks, warps, nitems,
+                     s);
+    const cudaError_t e = PrepareResident<T>(halves, ranks);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&c.cfg, ResidentKernelOf<T>(halves), bd, pc,
+                              items, steps, macro ? 1 : 0, src, dst);
+}
+
+template <typename T>
+bool BatchResidentLaunch<T>::Held(int halves, int ranks) {
+    ResidentConfig c(ResidentSmem(sizeof(T) == 8, halves), ranks, 24 >> halves,
+                     1, nullptr);
+    int clusters = 0;
+    if (PrepareResident<T>(halves, ranks) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, ResidentKernelOf<T>(halves),
+                                       &c.cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
+}
 
 }  // namespace mplb
