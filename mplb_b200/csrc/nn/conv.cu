@@ -654,7 +654,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     uint8_t* smem = Align1024(smem_raw);
     const int slices = a.bn / 32;
     const uint32_t stage_bytes = a.x_bytes + slices * a.dy_bytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + WgradBandData(a));
+    uint64_t* full = reinterpret_cast<uint64_t*>(
+        smem + WgradBandData(a.stages, a.x_bytes, a.dy_bytes, a.bn));
     uint64_t* empty = full + a.stages;
     uint64_t* accum = empty + a.stages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
@@ -1101,51 +1102,28 @@ bool LaunchConv(const View& x, const void* w, int taps, const float* bias,
 
 bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
                      cudaStream_t stream, int* err_dev, std::string& err) {
+    const WgradBandPlan p =
+        PlanWgradBand(x.nimg, x.h, x.w, x.c, dy.c, sm_count);
+    if (p.rows == 0) {
+        err = "weight gradient: a row does not fit in shared memory";
+        return false;
+    }
     WgradBandArgs a{};
     a.w = x.w;
     a.h = x.h;
     a.pitch = x.w + 2;
     a.cout = dy.c;
     a.cin = x.c;
-    a.bn = 32 * std::min(4, (dy.c + 31) / 32);
-    const int slices = (x.c + 31) / 32, groups = (dy.c + a.bn - 1) / a.bn;
-    a.stages = 2;
-    // as many rows as leave room for two stages (a band reads two rows more
-    // than it has), and a band at least for every CTA: one CTA per SM (a
-    // training step, with an atomic per lane, 535 us in these kernels, with two
-    // per SM 701), and as many again for each further group of output channels,
-    // whose layers have few pixels: 256 -> 256 at 16^2 adds up 512 products per
-    // accumulator as tap by tap (2.9e-7 off the 64-bit sums); with 1024 it were
-    // 6.4e-7.  A CTA has at least 128 pixels to pay for its sums' way out.
-    const int per_slice = std::max(
-        1, (int)std::min<long long>(sm_count / slices,
-                                    (long long)x.nimg * x.h * x.w / 128));
-    a.rows = std::min(x.h, 250);
-    const auto fits = [&] {
-        a.x_bytes = WgradBandBytes((a.rows + 2) * a.pitch + 3);
-        a.dy_bytes = WgradBandBytes(a.rows * a.pitch);
-        return WgradBandSmemBytes(a) <= kSmemMax;
-    };
-    while (a.rows > 1 &&
-           (!fits() ||
-            (long long)x.nimg * ((x.h + a.rows - 1) / a.rows) < per_slice))
-        a.rows--;
-    if (!fits()) {
-        err = "weight gradient: a row does not fit in shared memory";
-        return false;
-    }
-    while (a.stages < 4) {
-        a.stages++;
-        if (WgradBandSmemBytes(a) > kSmemMax) {
-            a.stages--;
-            break;
-        }
-    }
+    a.bn = p.bn;
+    a.rows = p.rows;
+    a.stages = p.stages;
+    a.x_bytes = WgradBandBytes((a.rows + 2) * a.pitch + 3);
+    a.dy_bytes = WgradBandBytes(a.rows * a.pitch);
     a.x_box = (uint32_t)((a.rows + 2) * a.pitch * 64);
     a.dy_box = (uint32_t)(a.rows * a.pitch * 64);
-    a.bands_per_img = (x.h + a.rows - 1) / a.rows;
+    a.bands_per_img = p.bands_per_img;
     a.bands_total = x.nimg * a.bands_per_img;
-    a.bands_per_cta = (a.bands_total + per_slice - 1) / per_slice;
+    a.bands_per_cta = p.bands_per_cta;
     a.tmem_cols = Pow2Cols(3 * a.bn);
     a.dw = dw;
     a.err = err_dev;
@@ -1157,9 +1135,9 @@ bool LaunchWgradBand(const View& dy, const View& x, float* dw, int sm_count,
     a.bulk = reinterpret_cast<uintptr_t>(dw) % 16 == 0 && x.c % 4 == 0 ? 1 : 0;
     if (a.bulk && !EncodeWeightGrad(&tdw, dw, x.c, dy.c, a.bn, err))
         return false;
-    const dim3 grid((a.bands_total + a.bands_per_cta - 1) / a.bands_per_cta,
-                    slices, groups);
-    const int smem = ResidencySafeSmem(WgradBandSmemBytes(a), a.tmem_cols);
+    const dim3 grid(p.ctas, p.slices, p.groups);
+    const int smem = ResidencySafeSmem(
+        WgradBandSmem(a.w, a.rows, a.stages, a.bn), a.tmem_cols);
     static cudaError_t attr = cudaFuncSetAttribute(
         WgradBandKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
     cudaError_t e = attr;
@@ -1208,11 +1186,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
         t.tmem_cols = Pow2Cols(t.bn);
         t.kb_total = x.nimg * t.tiles_per_img;
         const int mtiles = (t.n_atoms + 3) / 4;
-        int splits = (2 * sm_count + mtiles - 1) / mtiles;
-        if (splits < 1) splits = 1;
-        if (splits > t.kb_total) splits = t.kb_total;
-        t.kb_per_split = (t.kb_total + splits - 1) / splits;
-        splits = (t.kb_total + t.kb_per_split - 1) / t.kb_per_split;
+        t.kb_per_split = WgradTapBlocks(t.kb_total, taps, x.c, dy.c, sm_count);
+        const int splits = (t.kb_total + t.kb_per_split - 1) / t.kb_per_split;
         t.dw = dw;
         t.err = err_dev;
         const int smem = ResidencySafeSmem(WgradTSmemBytes(t.bn, t.stages),
@@ -1247,11 +1222,8 @@ bool LaunchWgrad(const View& dy, const View& x, int taps, float* dw,
     a.tmem_cols = Pow2Cols(a.bn);
     a.kb_total = x.nimg * a.tiles_per_img;
     const int blocks = taps * ((dy.c + 127) / 128) * ((x.c + a.bn - 1) / a.bn);
-    int splits = (2 * sm_count + blocks - 1) / blocks;
-    if (splits < 1) splits = 1;
-    if (splits > a.kb_total) splits = a.kb_total;
-    a.kb_per_split = (a.kb_total + splits - 1) / splits;
-    splits = (a.kb_total + a.kb_per_split - 1) / a.kb_per_split;
+    a.kb_per_split = WgradTapBlocks(a.kb_total, taps, x.c, dy.c, sm_count);
+    const int splits = (a.kb_total + a.kb_per_split - 1) / a.kb_per_split;
     a.dw = dw;
     a.err = err_dev;
     const int smem = ResidencySafeSmem(WgradSmemBytes(a.b_atoms, a.stages),

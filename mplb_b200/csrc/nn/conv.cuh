@@ -197,15 +197,6 @@ __global__ void WgradKernel(const __grid_constant__ CUtensorMap ta,
 inline int WgradSmemBytes(int b_atoms, int stages) {
     return 1024 + stages * ((2 + b_atoms) * 16384) + 256;
 }
-// The stages, in whose place the sums of three taps are laid out at the end.
-__host__ __device__ inline int WgradBandData(const WgradBandArgs& a) {
-    const int stages = a.stages * (a.x_bytes + a.bn / 32 * a.dy_bytes);
-    const int sums = 3 * a.bn * 32 * 4;
-    return stages > sums ? stages : sums;
-}
-inline int WgradBandSmemBytes(const WgradBandArgs& a) {
-    return 1024 + WgradBandData(a) + 256;
-}
 // WgradTKernel: per stage four 8 KiB X atoms and bn / 32 8 KiB dY atoms.
 inline int WgradTSmemBytes(int bn, int stages) {
     return 1024 + stages * ((4 + bn / 32) * 8192) + 256;

@@ -4,6 +4,12 @@
 
 #include <algorithm>
 
+#ifdef __CUDACC__
+#define MPLB_HD __host__ __device__
+#else
+#define MPLB_HD
+#endif
+
 namespace mplb {
 namespace nn {
 
@@ -172,17 +178,124 @@ inline BandPlan PlanBand(int nimg, int H, int W, int cin, int cout,
     return p;
 }
 
-// WgradBandKernel: a slice of so many positions.
-inline int WgradBandBytes(int positions) {
-    return (positions * 64 + 1023) / 1024 * 1024;
-}
-
 // Images narrower than this take the 3x3 weight gradient tap by tap.  A band
 // (WgradBandKernel) sums whole 16-position steps of one image row; a narrower
 // row would fill up its step with the row's two halo columns and the next row,
 // where a zero of dY meets a pixel of X that the tap does not use, and an
 // infinity or NaN there would enter the tap's sum.
 constexpr int kWgradBandWidth = 16;
+
+// WgradBandKernel: shared memory of a slice of so many positions; of the stages,
+// in whose place the sums of three taps are laid out at the end; of a launch.
+inline int WgradBandBytes(int positions) {
+    return (positions * 64 + 1023) / 1024 * 1024;
+}
+MPLB_HD inline int WgradBandData(int stages, int x_bytes, int dy_bytes,
+                                 int bn) {
+    const int ring = stages * (x_bytes + bn / 32 * dy_bytes);
+    const int sums = 3 * bn * 32 * 4;
+    return ring > sums ? ring : sums;
+}
+inline int WgradBandSmem(int w, int rows, int stages, int bn) {
+    const int pitch = w + 2;
+    return 1024 + 256 +
+           WgradBandData(stages, WgradBandBytes((rows + 2) * pitch + 3),
+                         WgradBandBytes(rows * pitch), bn);
+}
+
+// 128-pixel blocks that one accumulator of the tap-by-tap weight gradients sums
+// (WgradTKernel up to 64 output channels, WgradKernel above): two CTAs per SM.
+inline int WgradTapBlocks(long long blocks, int taps, int cin, int cout,
+                          int sm_count) {
+    long long tiles;   // of M and N, split `splits` times over the blocks
+    if (cout <= 64) {
+        tiles = (taps * ((cin + 31) / 32) + 3) / 4;
+    } else {
+        const int bn = 64 * std::min(4, (cin + 63) / 64);
+        tiles = (long long)taps * ((cout + 127) / 128) * ((cin + bn - 1) / bn);
+    }
+    const long long splits = std::max(
+        1LL, std::min((2LL * sm_count + tiles - 1) / tiles, blocks));
+    return (int)((blocks + splits - 1) / splits);
+}
+
+// How a 3x3 weight gradient is cut into bands of image rows.
+struct WgradBandPlan {
+    int bn = 0;              // output channels of a CTA
+    int slices = 0;          // of 32 input channels
+    int groups = 0;          // of bn output channels
+    int rows = 0;            // of a band; 0: no plan
+    int bands_per_img = 0;
+    int bands_per_cta = 0;
+    int ctas = 0;            // of a slice and group
+    int stages = 0;
+};
+
+// One CTA is on an SM at a time (a training step, with an atomic per lane, 535
+// us in these kernels, with two per SM 701).  Every height of bands that fits is
+// tried with every number of rounds of CTAs, and the shortest launch taken: a
+// round takes about 4.5 us and 1 ns for each 30 bytes of its CTAs' operands (a
+// band reads two rows more than it has), fitted to 32 and 64 images of the
+// network's layers.  Heights are even over an image (16 rows are two bands of 8,
+// never 15 and 1), and a CTA has at least 128 pixels to pay for its sums' way
+// out.
+//
+// A CTA sums its pixels in one fp32 accumulator, and the error against 64-bit
+// sums grows with their number.  So it sums no more than the tap-by-tap kernels
+// do (384 -> 128 at 32^2, 32 images: 1.38e-6 off with their 2,048 pixels, 1.97e-6
+// with 2,912), and no more than twice an SM's share of one group of output
+// channels (256 -> 256 at 16^2: 2.9e-7 with 512 pixels, 6.4e-7 with 1,024).
+inline WgradBandPlan PlanWgradBand(int nimg, int h, int w, int cin, int cout,
+                                   int sm_count) {
+    WgradBandPlan p;
+    p.bn = 32 * std::min(4, (cout + 31) / 32);
+    p.slices = (cin + 31) / 32;
+    p.groups = (cout + p.bn - 1) / p.bn;
+    const long long pixels = (long long)nimg * h * w;
+    const long long share = 2 * pixels * p.slices / sm_count;
+    const long long most = std::min<long long>(
+        128LL * WgradTapBlocks(pixels / 128, 9, cin, cout, sm_count),
+        std::max(128LL, share));
+    const long long planes = (long long)p.slices * p.groups;
+    double best = 0;
+    for (int rows = std::min(h, 250); rows >= 1; rows--) {
+        const int per_img = (h + rows - 1) / rows;
+        if ((h + per_img - 1) / per_img != rows ||
+            WgradBandSmem(w, rows, 2, p.bn) > kSmemMax)
+            continue;
+        const long long bands = (long long)nimg * per_img;
+        const long long band = (long long)rows * w;
+        if (band > most) continue;
+        const long long fewest = std::min(bands, (127 + band) / band);
+        // rounds: from the first in which no CTA has more than `most` pixels
+        const long long first = (bands + most / band - 1) / (most / band);
+        long long rounds = (first * planes + sm_count - 1) / sm_count;
+        for (int tries = 0; tries < 3; tries++, rounds++) {
+            const long long ctas = rounds * sm_count / planes;
+            const long long per =
+                std::max(fewest, (bands + ctas - 1) / std::max(1LL, ctas));
+            if (ctas < 1 || per * band > most) continue;
+            const long long used = (bands + per - 1) / per;
+            const double time =
+                (double)((used * planes + sm_count - 1) / sm_count) *
+                    ((double)(per * band) *
+                         (64.0 * (rows + 2) / rows + 2.0 * p.bn) / 30 +
+                     4500) +
+                (double)used * 1e-3;
+            if (p.rows != 0 && time >= best) continue;
+            best = time;
+            p.rows = rows;
+            p.bands_per_img = per_img;
+            p.bands_per_cta = (int)per;
+            p.ctas = (int)used;
+        }
+    }
+    p.stages = 2;
+    while (p.rows != 0 && p.stages < 4 &&
+           WgradBandSmem(w, p.rows, p.stages + 1, p.bn) <= kSmemMax)
+        p.stages++;
+    return p;
+}
 
 }  // namespace nn
 }  // namespace mplb

@@ -18,6 +18,14 @@ int main() {
     while (scanf("%15s %d %d %d %d %d", what, &n, &h, &w, &cin, &cout) == 6)
         if (!strcmp(what, "band"))
             printf("%d\n", PlanBand(n, h, w, cin, cout, 148).tiles);
+        else {
+            const WgradBandPlan p = PlanWgradBand(n, h, w, cin, cout, 148);
+            printf("%d %d %d %d %d %d %d %d %d %d\n", p.bn, p.slices, p.groups,
+                   p.rows, p.bands_per_img, p.bands_per_cta, p.ctas, p.stages,
+                   WgradBandSmem(w, p.rows, p.stages, p.bn),
+                   128 * WgradTapBlocks((long long)n * h * w / 128, 9, cin,
+                                        cout, 148));
+        }
 }
 """
 
@@ -65,3 +73,44 @@ def test_the_faster_form_is_taken(ask):
 
 def test_wide_inputs_go_tap_by_tap(ask):
     assert ask("band", [(32, 64, 64, 144, 64), (1, 16, 16, 384, 16)]) == [[0]] * 2
+
+
+WGRAD = [(n, h, w, ci, co)
+         for n in (1, 2, 3, 5, 8, 20, 32, 64, 100)
+         for h, w in ((16, 16), (24, 16), (32, 32), (36, 32), (64, 64), (6, 64),
+                      (128, 128), (1, 128), (9, 128), (1000, 32))
+         for ci, co in ((32, 32), (96, 32), (16, 48), (32, 64), (64, 64),
+                        (192, 64), (64, 128), (128, 128), (384, 128),
+                        (128, 256), (256, 256), (5000, 16))]
+
+
+def test_weight_gradient_bands(ask):
+    """Bands cover every image in even heights, fit in shared memory, and no
+    accumulator sums more pixels than those of the tap-by-tap kernels (their
+    fp32 error grows with the number), or than twice an SM's share of a group
+    of output channels."""
+    for shape, got in zip(WGRAD, ask("wgrad", WGRAD)):
+        n, h, w, ci, co = shape
+        bn, slices, groups, rows, per_img, per_cta, ctas, stages, smem, tap = got
+        assert bn * groups >= co and 32 * slices >= ci
+        assert rows >= 1 and per_img == -(-h // rows), shape
+        assert rows == -(-h // per_img) and rows <= 250
+        assert ctas == -(-n * per_img // per_cta)
+        assert 2 <= stages <= 4 and smem <= 227 * 1024
+        assert rows * per_cta * w <= tap, shape
+        share = 2 * n * h * w * slices // 148
+        assert rows * per_cta * w <= max(128, share), shape
+        # enough pixels to pay for the sums' way out, where there are any
+        assert rows * per_cta * w >= min(128, n * h * w), shape
+
+
+def test_weight_gradients_fill_the_gpu(ask):
+    """The network's layers at 32 and 8 images: CTAs for nine tenths of the
+    SMs, or of the last round of them."""
+    layers = [(128, 32, 32), (128, 96, 32), (64, 32, 64), (64, 64, 64),
+              (64, 192, 64), (32, 128, 128), (32, 384, 128)]
+    shapes = [(n, s, s, ci, co) for n in (8, 32) for s, ci, co in layers]
+    for shape, got in zip(shapes, ask("wgrad", shapes)):
+        ctas = got[6] * got[1] * got[2]
+        rounds = -(-ctas // 148)
+        assert ctas >= 0.85 * 148 * rounds, (shape, ctas)
