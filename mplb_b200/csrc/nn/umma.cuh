@@ -107,15 +107,15 @@ __device__ __forceinline__ void Mma(uint32_t d_tmem, uint64_t a_desc,
 // operands (uniform registers) directly, where behind a test of the lane
 // number each MMA took over 100 cycles to issue.
 __device__ __forceinline__ bool ElectOne() {
-    uint32_t pred = 0, lane = 0;
+    uint32_t chosen;   // elect.sync sets its predicate in one lane of the mask
     asm volatile(
-        "{\n\t.reg .b32 %%rx;\n\t.reg .pred %%px;\n\t"
-        "elect.sync %%rx|%%px, %2;\n\t"
-        "@%%px mov.s32 %1, 1;\n\t"
-        "mov.s32 %0, %%rx;\n\t}"
-        : "+r"(lane), "+r"(pred)
-        : "r"(0xFFFFFFFFu));
-    return pred != 0;
+        "{\n\t"
+        ".reg .pred one;\n\t"
+        "elect.sync _|one, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, one;\n\t"
+        "}"
+        : "=r"(chosen));
+    return chosen != 0;
 }
 
 // The same with the descriptors' two words apart (the high one, SmemDescHigh,
