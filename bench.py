@@ -380,7 +380,7 @@ def run_cavities(args, rank, world, local):
                              "through HBM; steps of one call run in shared "
                              "memory",
                      "traffic": None},
-        "tuning": tuned["tuning"],
+        "tuning": dict(tuned["tuning"], route=tuned["route"]),
         "autotune": [{"mlups": round(r["mlups"], 1),
                       **{k: v for k, v in r.items() if k != "mlups"}}
                      for r in tuned["all"]],

@@ -322,13 +322,20 @@ typedef struct {
     double tau_ref;  /* MPLB tauRef (tau_L = tauRef / dt + 1/2) */
 } mplbgpu_cavity;
 
+/* How a batch steps.  With persistent = 0, a call's steps (mplbgpu_batch_step,
+ * or a check period of mplbgpu_batch_run) from four on advance strips of the
+ * cavities in shared memory, many steps a launch, while every active cavity
+ * has at most 800 nodes a side (400 in FP64) and the device holds the strips'
+ * clusters; nothing below changes those launches.  The other cases take the
+ * launches described here. */
 typedef struct {
     int tile_nodes;  /* nodes per tile: 64, 128 or 256; a CTA has one
                         thread per node in FP64 and one per two nodes in
                         FP32 */
     int persistent;  /* 1: one cooperative launch per chunk of steps with a
                         bounded grid barrier between steps; 0: one launch
-                        per step, a chunk replayed from a CUDA graph */
+                        per step, a chunk replayed from a CUDA graph, where
+                        the steps do not stay in shared memory (above) */
     int chunk;       /* steps per chunk (even) */
     int ctas_per_sm; /* CTAs per SM of the persistent launches (at most
                         the co-resident count) */

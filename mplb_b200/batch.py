@@ -14,7 +14,8 @@ the cavities are independent, so there is no data-path exchange).
 ``Batch`` wraps one batch on the GPU; ``autotune`` times tile size, launch
 style (CUDA-graph chunks of one-step launches or a persistent multi-step
 launch), CTAs per SM and chunk length on the batch itself and caches the
-winner in a JSON file keyed by device, precision and the cavity sizes.
+winner in a JSON file keyed by device, precision, the cavity sizes and the
+sources of the batch's kernels.
 """
 import ctypes
 import dataclasses
@@ -240,6 +241,18 @@ class Batch:
                     launches=nl.value)
 
 
+def _kernel_build() -> str:
+    """Digest of the sources that make up the batch's kernels and the choice
+    among them: a tuning measured with others says nothing about these."""
+    csrc = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
+    h = hashlib.sha1()
+    for name in sorted(os.listdir(csrc)):
+        if name.startswith("batch") or name in ("kernels.cuh", "lattice.h"):
+            with open(os.path.join(csrc, name), "rb") as fh:
+                h.update(name.encode() + fh.read())
+    return h.hexdigest()[:12]
+
+
 def _cache_key(batch: Batch) -> str:
     import torch
     name = torch.cuda.get_device_name() if torch.cuda.is_available() else "?"
@@ -247,12 +260,14 @@ def _cache_key(batch: Batch) -> str:
     for s in batch.specs:
         hist[s.n] = hist.get(s.n, 0) + 1
     h = hashlib.sha1(json.dumps(sorted(hist.items())).encode()).hexdigest()
-    return f"{name}|{batch.precision}|{h[:12]}"
+    return f"{name}|{batch.precision}|{h[:12]}|{_kernel_build()}"
 
 
 def default_candidates():
     """Tile size x launch style: one CTA per tile (persistent 0) or
-    cooperative persistent steps (1, x CTAs per SM)."""
+    cooperative persistent steps (1, x CTAs per SM).  The tile size of
+    persistent 0 matters for batches with a side too large to stay in shared
+    memory, and for calls of fewer than four steps."""
     graph = [dict(tile_nodes=t, persistent=0, chunk=50, ctas_per_sm=8)
              for t in (64, 128, 256)]
     persistent = [dict(tile_nodes=t, persistent=1, chunk=50, ctas_per_sm=k)
@@ -263,7 +278,11 @@ def default_candidates():
 def autotune(batch: Batch, steps: int = 200, cache: str = DEFAULT_CACHE,
              candidates=None, force=False):
     """Times each candidate tuning on `batch` (from its initial state) and
-    keeps the fastest (MLUPS over `steps` steps); results are cached."""
+    keeps the fastest (MLUPS over `steps` steps); results are cached by
+    device, precision, sides and kernels.  Each result names its `route`:
+    "resident" (many steps a launch in shared memory), "steps" (a launch each)
+    or "persistent".  Resident launches are the same under every tuning, so
+    they are timed once and the first such candidate stands for them."""
     key = _cache_key(batch)
     table = {}
     if os.path.exists(cache):
@@ -275,7 +294,11 @@ def autotune(batch: Batch, steps: int = 200, cache: str = DEFAULT_CACHE,
     if candidates is None:
         candidates = default_candidates()
     results = []
+    resident = None
     for cand in candidates:
+        if resident is not None and not cand.get("persistent", 0):
+            results.append((resident, cand, "resident"))
+            continue
         batch.set_tuning(**cand)
         batch.init()
         batch.step(cand["chunk"])            # warm-up (graph capture)
@@ -284,10 +307,14 @@ def autotune(batch: Batch, steps: int = 200, cache: str = DEFAULT_CACHE,
         s1 = batch.stats()
         ms = s1["device_ms"] - s0["device_ms"]
         mlups = batch.total_nodes * steps / (ms * 1e-3) / 1e6
-        results.append((mlups, cand))
-    results.sort(key=lambda r: -r[0])
+        route = "persistent" if cand.get("persistent", 0) else "steps"
+        if route == "steps" and s1["launches"] - s0["launches"] < steps:
+            route, resident = "resident", mlups
+        results.append((mlups, cand, route))
+    results.sort(key=lambda r: -r[0])        # stable: the first of equals
     best = {"tuning": results[0][1], "mlups": results[0][0],
-            "all": [{"mlups": m, **c} for m, c in results]}
+            "route": results[0][2],
+            "all": [{"mlups": m, "route": r, **c} for m, c, r in results]}
     table[key] = best
     with open(cache, "w") as fh:
         json.dump(table, fh, indent=1)
