@@ -304,8 +304,9 @@ mplbgpu_status mplbgpu_synchronize(mplbgpu_ctx* ctx);
 /* Number of kernel launches the context has issued since creation. */
 long long mplbgpu_launch_count(const mplbgpu_ctx* ctx);
 
-/* Device time of the most recent mplbgpu_step call's kernels (ms); waits
- * for them to finish. */
+/* Device time of the most recent mplbgpu_step call's kernels (ms), from the
+ * call, or from the end of the previous step call's kernels where those still
+ * ran, to their own end; waits for it. */
 mplbgpu_status mplbgpu_last_step_ms(mplbgpu_ctx* ctx, float* ms);
 
 /* ---------------------------------------------------------------------

@@ -4,7 +4,7 @@
 // blocks beyond the L2 cache ran at 80-83 % of the copy peak.  Here a CTA
 // takes a tile of 256 bytes by kTileH rows of nodes, computes the first step
 // on the tile and one node around it (10-14 % more nodes) into shared memory,
-// and the second step from there, so two steps move the populations once: 263
+// and the second step from there, so two steps move the populations once: 302
 // MB read and written for two FP32 steps of 4096 x 1024 nodes, where single
 // steps move 604.  A node's 193 warp instructions per 32 nodes and step (index
 // arithmetic a third of them) and their waits at 24 warps per SM are the bound

@@ -845,12 +845,14 @@ __device__ __forceinline__ void ApplyWallOps(typename Prec<T>::C* f,
     }
 }
 
-// A kernel of a step launched over the tail of the one before it
-// (programmatic stream serialisation, LaunchOver): its CTAs may take their
-// places as that one's end, and wait here for its results.  Nothing in an
-// ordinary launch.  (Letting them start as soon as all of that one's CTAs have
-// started filled the free places unevenly: 64^3 in FP16 15.0 us a step against
-// 11.3, 24^3 in FP32 6.1 against 4.9.)
+// A kernel of a step launched with programmatic stream serialisation
+// (LaunchOver) waits here for the results of the one before it.  No kernel
+// triggers its successor early, so that one's CTAs come in when the last CTA of
+// this one has ended: what the attribute saves is the launch, which no longer
+// waits for this one's results to be flushed.  Nothing in an ordinary launch.
+// (An early trigger, griddepcontrol.launch_dependents at the start of a CTA,
+// filled the free places unevenly: 64^3 in FP16 15.0 us a step against 11.3,
+// 24^3 in FP32 6.1 against 4.9.)
 __device__ __forceinline__ void WaitForPrevious() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -1389,8 +1391,10 @@ __device__ __forceinline__ void CpAsyncWait() {
 }
 
 // The staged interior of one CTA of a chunk (see StagedStep): warp k takes
-// the chunk's tasks (w - 1) kSplitWarps tasks + k tasks + t, t < tasks (task -> row t / tasks per row, segment t % tasks per
-// row).  Lane l computes the pair l, l + 32 of the segment (PairFinish).
+// `tasks` of the chunk's 64-node segments, numbers
+// ((w - 1) kSplitWarps + k) tasks and on (number g is segment g % s of row
+// g / s, s segments to a row).  Lane l computes the pair l, l + 32 of the
+// segment (PairFinish).
 template <int D, typename T, bool O32>
 __device__ __forceinline__ void StagedInterior(const BlockDev& b,
                                                const PhysConst& pc,
@@ -1506,7 +1510,8 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value
     const unsigned nsr = (unsigned)nbx * (2 * nz + (D == 3 ? 2 * ny : 0));
     constexpr int G = SplitGroup<T>();
     constexpr bool kStaged = StagedStep<T>();
-    const unsigned per_chunk = (unsigned)SplitChunkCtas<G, kStaged>(b.n[0], tasks);
+    const unsigned per_chunk =
+        (unsigned)SplitChunkCtas<G, kStaged>(b.n[0], tasks);
     // CTA order: spc = 0, the shell rows first, then the chunks (blk0: a
     // launch of the chunks alone starts after the shell rows);
     // spc = kWallsFirst, the shell rows, every chunk's x-face CTA, then the

@@ -12,8 +12,9 @@ namespace mplb {
 
 template <int D, typename T>
 struct Launch {
-    // `over` (here and below): a kernel of a step that may start over the
-    // tail of the one queued before it on the stream, itself one of these
+    // `over` (here and below): a kernel of a step that is admitted when the
+    // last CTA of the one queued before it on the stream, itself one of these,
+    // has ended
     static cudaError_t Step(int mode, bool over, dim3 grid, cudaStream_t s,
                             const BlockDev& b, const PhysConst& pc,
                             const T* src, T* dst, double* o0, double* o1,

@@ -37,10 +37,11 @@ long long SplitShellBlocks(const BlockDev& b) {
     return nbx * (2 * nz + (D == 3 ? 2 * ny : 0));
 }
 
-// Launches `kernel`, with `over` allowed to start over the tail of the kernel
-// queued before it on the stream (every such kernel begins with
-// WaitForPrevious).  Between two steps that saves the launch of the second:
-// 32^3 in FP64 8.2 -> 6.1 us a step, 64^3 16.8 -> 14.8, 256^3 850 -> 825.
+// Launches `kernel`, with `over` admitted as soon as the last CTA of the kernel
+// queued before it on the stream has ended, before that one's results are
+// flushed (every such kernel begins with WaitForPrevious).  Between two steps
+// that hides the launch of the second: 32^3 in FP64 6.1 us a step against 8.2,
+// 64^3 14.8 against 16.8, 256^3 825 against 850.
 template <typename... P, typename... A>
 cudaError_t LaunchOver(bool over, void (*kernel)(P...), dim3 grid,
                        unsigned threads, int smem, cudaStream_t s,

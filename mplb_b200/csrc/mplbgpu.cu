@@ -350,8 +350,8 @@ int SwapStepOnce(mplbgpu_ctx* ctx, bool over) {
 // over the context's stream and its side streams (forked after the previous
 // step's halos, joined before this step's), so that one launch's tail
 // overlaps the next one's start.  A step on one stream that follows another of
-// the same call (`over`) starts over that one's tail, and its halos over its
-// own.
+// the same call (`over`) is admitted as that one's last CTA ends, and its halos
+// as its own does.
 template <int D, typename T>
 int StepOnce(mplbgpu_ctx* ctx, bool over) {
     if (ctx->plan.swap) return SwapStepOnce<D, T>(ctx, over);
@@ -375,8 +375,9 @@ int StepOnce(mplbgpu_ctx* ctx, bool over) {
         const T* s = static_cast<const T*>(b.pop[src]);
         T* d = static_cast<T*>(b.pop[dst]);
         CK_LAUNCH_E(Launch<D, T>::Step(kModeStep, over && lanes == 1,
-                                       NodeGrid(B, D), next(), b.dev, ctx->pc, s, d, nullptr, nullptr,
-                                       nullptr, nullptr));
+                                       NodeGrid(B, D), next(), b.dev, ctx->pc,
+                                       s, d, nullptr, nullptr, nullptr,
+                                       nullptr));
         if (B.ndeferred > 0 && b.dev.deferred_fused) {
             const unsigned g = (unsigned)((B.ndeferred + kThreads - 1) / kThreads);
             CK_LAUNCH_E(Launch<D, T>::DeferredFused(g, next(), b.dev, ctx->pc,
@@ -550,10 +551,10 @@ int Observe(mplbgpu_ctx* ctx, int mode, size_t bi, double* o0, double* o1,
     const BlockPlan& B = ctx->plan.blocks[bi];
     if (ctx->plan.swap) {
         const int st = ctx->swap_state;
-        CK_LAUNCH_E(Launch<D, T>::Swap(mode, false, st == 1, st != 0, NodeGrid(B, D),
-                                       ctx->stream, b.dev, ctx->pc,
-                                       static_cast<T*>(b.pop[0]), o0, o1, o2,
-                                       o3));
+        CK_LAUNCH_E(Launch<D, T>::Swap(mode, false, st == 1, st != 0,
+                                       NodeGrid(B, D), ctx->stream, b.dev,
+                                       ctx->pc, static_cast<T*>(b.pop[0]), o0,
+                                       o1, o2, o3));
         return MPLBGPU_OK;
     }
     const int prev = 1 - ctx->cur;
@@ -564,8 +565,9 @@ int Observe(mplbgpu_ctx* ctx, int mode, size_t bi, double* o0, double* o1,
                                                 pv, o0, o1, o2, o3));
         return MPLBGPU_OK;
     }
-    CK_LAUNCH_E(Launch<D, T>::Step(mode, false, NodeGrid(B, D), ctx->stream, b.dev,
-                                   ctx->pc, pv, nullptr, o0, o1, o2, o3));
+    CK_LAUNCH_E(Launch<D, T>::Step(mode, false, NodeGrid(B, D), ctx->stream,
+                                   b.dev, ctx->pc, pv, nullptr, o0, o1, o2,
+                                   o3));
     if (B.ndeferred > 0) {
         const unsigned g = (unsigned)((B.ndeferred + kThreads - 1) / kThreads);
         CK_LAUNCH_E(Launch<D, T>::DeferredFinish(mode, g, ctx->stream, b.dev,

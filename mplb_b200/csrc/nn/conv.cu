@@ -756,11 +756,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     if (!acc_ok && threadIdx.x == 0) Flag(cta_err, a.err);
     const bool store = __all_sync(~0u, acc_ok && *cta_err == 0);
     // TMEM lane 32 w + c: tap column w (the fourth belongs to no tap).  The
-    // stages are read by now: each warp lays its tap's 32 x bn sums out there and
-    // one bulk reduction adds them to dW, clipped at its edges.  Lane by lane, at
-    // about one atomic a cycle and SM, this took most of the layers of few pixels
-    // and many channels: 256 -> 256 at 16^2 56 us
-    // -> 34, a training step 535 us in this kernel -> 413.
+    // stages are read by now: each warp lays its tap's 32 x bn sums out there,
+    // and one bulk reduction adds them to dW, clipped at its edges.  Lane by
+    // lane, at about one atomic a cycle and SM, this took most of the layers of
+    // few pixels and many channels: 256 -> 256 at 16^2 56 us, in bulk 34.
     const int ci = c0 + lane;
     const uint32_t row = tmem + ((uint32_t)(warp * 32) << 16);
     float* out = reinterpret_cast<float*>(smem) + warp * a.bn * 32;

@@ -34,8 +34,8 @@
 //
 // The weight gradient of a 3x3 convolution over rows of 16 pixels or more is
 // WgradBandKernel's (below); the two that follow serve narrower rows and 1x1
-// convolutions.  WgradKernel computes dW[n][t][c] += sum over pixels p of dY[p][n] *
-// X[p + offset(t)][c]: M = 128 output channels, N = input channels, K = a
+// convolutions.  WgradKernel computes dW[n][t][c] += sum over pixels p of
+// dY[p][n] * X[p + offset(t)][c]: M = 128 output channels, N = input channels, K = a
 // range of 128-pixel blocks (split over CTAs, accumulated with fp32 atomics).
 // Both operands arrive pixel-major with channels contiguous, i.e. MN-major,
 // as 64-channel TMA boxes swizzled by 128 bytes.
@@ -146,13 +146,13 @@ struct WgradTArgs {
 
 // Weight gradient of a 3x3 convolution with its operands resident: a band of
 // image rows of one 32-channel slice of X (with its halo) and of bn channels of
-// dY in shared memory serve all nine taps.  Both are laid out W + 2 positions to
-// a row, and tap (dh, dw) pairs dY's position q with X's position
-// q + dh (W + 2) + dw, for the W positions of each row.  M = 128 rows are the slice at four consecutive dw - three
-// of them taps: the operand descriptor steps one position between its 32-row
-// atoms - N = the output channels, one accumulator per dh.  CTAs sum ranges of
-// bands and add them to dW in fp32 (bulk reductions).  Tap by tap X moved nine times through L2
-// for it.
+// dY in shared memory serve all nine taps (tap by tap X moved nine times through
+// L2).  Both are laid out W + 2 positions to a row, and tap (dh, dw) pairs dY's
+// position q with X's position q + dh (W + 2) + dw, for the W positions of each
+// row.  M = 128 rows are the slice at four consecutive dw - three of them taps:
+// the operand descriptor steps one position between its 32-row atoms - N = the
+// output channels, one accumulator per dh.  CTAs sum ranges of bands and add
+// them to dW in fp32 (bulk reductions).
 struct WgradBandArgs {
     int w, h;              // image
     int pitch;             // positions per row: W + 2
