@@ -75,10 +75,13 @@ bool WallsFirst(const BlockDev& b, int q) {
 template <int D, typename T>
 int StageTasks(const BlockDev& b) {
     if (!StagedStep<T>()) return 1;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long segments = (long long)(b.n[1] - 2) *
                                (D == 3 ? b.n[2] - 2 : 1) *
                                ((b.n[0] + 63) / 64);
-    const long long warps = 148 * MPLB_LP_MIN_BLOCKS * kSplitWarps;
+    const long long warps = (long long)sms * MPLB_LP_MIN_BLOCKS * kSplitWarps;
     int tasks = 1;
     while (tasks < kStageTasks && segments > tasks * warps) tasks *= 2;
     return tasks;
