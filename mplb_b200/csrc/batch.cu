@@ -66,7 +66,10 @@ struct mplbgpu_batch {
     ResidentItem* items = nullptr;
     size_t items_cap = 0;
     int sms = 1;
+    // what the device holds; a form and cluster size is taken for held until
+    // a plan first uses it and the device is asked
     ResidentHeld held;
+    bool asked[3][kNumResidentRanks] = {};
     static constexpr int kSides = 5;   // side streams of the classes, made
                                        // when a plan first needs them
     cudaStream_t side[kSides] = {};
@@ -151,7 +154,19 @@ int BuildResident(mplbgpu_batch* b) {
         sides.push_back(b->cav[c].n);
         base.push_back((int)(b->hcav[c].base / unit));
     }
-    b->resident = PlanStrips(b->active, sides, base, f64, b->sms, b->held);
+    for (bool replan = true; replan;) {
+        b->resident = PlanStrips(b->active, sides, base, f64, b->sms, b->held);
+        replan = false;
+        for (const ResidentClass& k : b->resident) {
+            const int r = ResidentRankIndex(k.ranks);
+            if (b->asked[k.halves][r]) continue;
+            b->asked[k.halves][r] = true;
+            b->held.at[k.halves][r] =
+                f64 ? BatchResidentLaunch<double>::Held(k.halves, k.ranks)
+                    : BatchResidentLaunch<float>::Held(k.halves, k.ranks);
+            replan = replan || !b->held.at[k.halves][r];
+        }
+    }
     std::vector<ResidentItem> all;
     for (const ResidentClass& k : b->resident)
         all.insert(all.end(), k.items.begin(), k.items.end());
@@ -528,12 +543,6 @@ mplbgpu_status mplbgpu_batch_create(const mplbgpu_cavity* cavities, int ncav,
     int dev = 0;
     CRE(cudaGetDevice(&dev));
     CRE(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev));
-    for (int h = 0; h < 3; h++)
-        for (int r = 0; r < kNumResidentRanks; r++)
-            b->held.at[h][r] =
-                precision == MPLBGPU_FP64
-                    ? BatchResidentLaunch<double>::Held(h, kResidentRanks[r])
-                    : BatchResidentLaunch<float>::Held(h, kResidentRanks[r]);
     CRE(cudaMalloc(&b->dcav, ncav * sizeof(BatchCav)));
     CRE(cudaMemcpy(b->dcav, b->hcav.data(), ncav * sizeof(BatchCav),
                    cudaMemcpyHostToDevice));

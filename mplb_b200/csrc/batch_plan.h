@@ -63,8 +63,16 @@ struct ResidentClass {
 // have no place for some that a whole B200 has.
 constexpr int kResidentRanks[] = {1, 2, 3, 4, 5, 6, 8, 9};
 constexpr int kNumResidentRanks = 8;
+inline int ResidentRankIndex(int ranks) {
+    int r = 0;
+    while (kResidentRanks[r] != ranks) r++;
+    return r;
+}
 struct ResidentHeld {
-    bool at[3][kNumResidentRanks] = {};   // [halves][index of the ranks]
+    bool at[3][kNumResidentRanks];   // [halves][index of the ranks]
+    ResidentHeld() {
+        for (auto& h : at) std::fill(h, h + kNumResidentRanks, true);
+    }
 };
 
 // How the cavities of one side are held in shared memory; score infinite: not
