@@ -98,8 +98,8 @@ inline double BandMicroseconds(const BandPlan& p, int pitch, int cin,
     const double mma =
         nkb * (bk / 16) * p.tiles * std::max(32.0, p.bn / 4.0) * 1e-3;
     const double input = (double)p.rows * pitch * bk * 2 * chunks * 1e-4;
-    return 3.9 + rounds * (1.1 * ((nkb + p.group - 1) / p.group) + 0.18 * mma) +
-           per * (0.35 * input + 0.014 * p.tiles * p.bn);
+    return 2.9 + rounds * (1.1 * ((nkb + p.group - 1) / p.group) + 0.24 * mma) +
+           per * (0.3 * input + 0.016 * p.tiles * p.bn);
 }
 
 // Tiles and output channels of a CTA (cold-L2 times of the network's layers, 32
