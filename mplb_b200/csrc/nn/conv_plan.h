@@ -67,8 +67,9 @@ struct BandPlan {
 };
 
 // Microseconds of a 3x3 convolution's launch, tap by tap and in bands, roughly:
-// fitted to the times (cold caches) of 1,696 shapes of 2,048 to 524,288 pixels,
-// rows of 1 to 128 pixels, 16 to 128 input and 16 to 384 output channels.
+// fitted to the times of 1,696 shapes with cold caches and 977 with the input in
+// L2: 2,048 to 524,288 pixels, rows of 1 to 128 pixels, 16 to 128 input and 16 to
+// 384 output channels.
 // `per` CTAs fall to the fullest SM, `rounds` one after the other.
 //
 // Tap by tap: a round's start, its k-blocks one behind the other (the loads'
@@ -108,12 +109,15 @@ inline double BandMicroseconds(const BandPlan& p, int pitch, int cin,
 // while the GPU is not full.  Above 128 input channels the
 // band fills the shared memory that the weights stream through (192 -> 64 at
 // 64^2 64 us, was 61; 384 -> 128 at 32^2 108, was 53).  Below, bands where they
-// take less time by the estimates above: they read the input once for at most
+// take no more time by the estimates above: they read the input once for at most
 // 128 output channels (tap by tap 256) and compute W + 2 columns of W, so that
 // 128 -> 256 at 16^2 takes 18 us in bands and 14 tap by tap (64 images 28 and
 // 14), 128 -> 384 at 32^2, 8 images, 19 and 14, 64 -> 64 at 32768 x 4 250 and
-// 220.  Of the 1,696 shapes the estimate picks the slower form by more than a
-// tenth in 39.
+// 220.  Within 4 % bands are taken: behind another launch of a pass they do
+// better than alone (predictions of 16 images 356 us with the 4 %, 361 without).
+// The choice is on average 0.8 % slower than the faster form with cold caches and
+// 0.6 % with the input in L2 (always bands 14 and 6 %, always tap by tap 10 and
+// 15 %), and by more than a tenth in 74 of the 2,673 shapes.
 inline BandPlan PlanBand(int nimg, int H, int W, int cin, int cout,
                          int sm_count) {
     BandPlan p;
@@ -173,7 +177,8 @@ inline BandPlan PlanBand(int nimg, int H, int W, int cin, int cout,
     }
     if (p.tiles > 0 &&
         BandMicroseconds(p, pitch, cin, sm_count) >=
-            TapMicroseconds((long long)nimg * H * W, cin, cout, sm_count))
+            1.04 * TapMicroseconds((long long)nimg * H * W, cin, cout,
+                                   sm_count))
         p.tiles = 0;
     return p;
 }
