@@ -639,8 +639,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 // The weight gradient of a 3x3 convolution (see conv.cuh): one 32-channel slice
 // of the input, bn output channels, a range of bands of image rows.  Cold-cache
 // layer times (32 images), tap by tap in brackets: 96 -> 32 at 128^2 61 us (202),
-// 32 -> 32 27 (77), 192 -> 64 at 64^2 43 (116), 384 -> 128 at 32^2 44 (78), 128 ->
-// 128 23 (43).  Row by row a sum has the terms of a tap's and no others: over
+// 32 -> 32 26 (77), 192 -> 64 at 64^2 43 (116), 384 -> 128 at 32^2 54 (78), 128 ->
+// 128 22 (43).  Row by row a sum has the terms of a tap's and no others: over
 // surplus columns, too, 256 -> 256 at 16^2 rounds 18/16 times as often, 3.0e-7 off
 // the 64-bit sums in place of 2.9e-7, and a pixel that a tap does not use enters it
 // times zero.  So rows are 16 pixels or a multiple (kWgradBandWidth).
